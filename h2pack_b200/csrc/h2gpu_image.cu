@@ -1834,7 +1834,7 @@ int run_panel(h2gpu_image* im, int NV, int nv, const double* X, long long x_rs, 
         CK(launch_jit(im->kernel_id, 1, NV, im->d_jtF2, im->n_jtF2, im->d_js, im->d_pts32, kp, 1, 1, im->d_XS,
                       im->d_PS, im->d_Y1, s, im->far_diff ? 0 : 1, im->d_ppts, im->d_pin, im->d_tiles, im->d_pts32lo,
                       im->d_pplo));
-        CK(launch_y1sum(NV, im->d_y1t2, im->n_y12, im->d_y1_slots2, im->d_PS, im->d_Y1, s));
+        CK(launch_y1sum(NV, im->d_y1t2, im->n_y12, im->d_y1_slots2, im->d_PS, im->d_Y1, im->y0_rows, s));
         if (timed) CK(cudaEventRecord(e[4], s));
         for (size_t L = 0; L + 1 < im->dn_beg.size(); L++)
         {
@@ -1842,7 +1842,8 @@ int run_panel(h2gpu_image* im, int NV, int nv, const double* X, long long x_rs, 
             CK(launch_down<float>(NV, im->d_dn + b, n, im->d_U32, im->d_Y1, im->d_PS, im->d_PUSH, s, sweep_tc(im)));
         }
         if (timed) CK(cudaEventRecord(e[5], s));
-        CK(launch_asm(NV, im->d_asm2, im->n_asm2, im->d_asm_slots2, im->d_PS, im->d_fwd, Y, y_rs, y_cs, nv, s));
+        CK(launch_asm(NV, im->d_asm2, im->n_asm2, im->d_asm_slots2, im->d_PS, im->d_fwd, Y, y_rs, y_cs, nv, im->N,
+                      s));
         if (timed) CK(cudaEventRecord(e[6], s));
         im->st.n_launches += 9 + (long long) (im->up_beg.size() - 1) + (long long) (im->dn_beg.size() - 1);
         return H2GPU_OK;
@@ -1901,7 +1902,7 @@ int run_panel(h2gpu_image* im, int NV, int nv, const double* X, long long x_rs, 
                                            im->blk1_small[0][1]));
         else CK(launch_blk<double>(NV, im->d_blkB, im->n_blkB, im->d_B64, im->d_XS, im->d_PS, s, 0, nullptr,
                                    im->blk1_small[0][0]));
-        CK(launch_y1sum(NV, im->d_y1t, im->n_y1, im->d_y1_slots, im->d_PS, im->d_Y1, s));
+        CK(launch_y1sum(NV, im->d_y1t, im->n_y1, im->d_y1_slots, im->d_PS, im->d_Y1, im->y0_rows, s));
     } else {
         const bool panels = f32 && panels_used(im, NV);
         if (panels) CK(launch_panel_in(NV, im->d_pg, im->n_pg_pts, im->n_pg - im->n_pg_pts, im->d_XS, im->d_pin, s));
@@ -1918,7 +1919,8 @@ int run_panel(h2gpu_image* im, int NV, int nv, const double* X, long long x_rs, 
         else CK(launch_down<double>(NV, im->d_dn + b, n, im->d_U64, im->d_Y1, im->d_PS, im->d_PUSH, s));
     }
     if (timed) CK(cudaEventRecord(e[5], s));
-    CK(launch_asm(NV, im->d_asm, im->n_asm, im->d_asm_slots, im->d_PS, im->d_fwd, Y, y_rs, y_cs, nv, s));
+    CK(launch_asm(NV, im->d_asm, im->n_asm, im->d_asm_slots, im->d_PS, im->d_fwd, Y, y_rs, y_cs, nv, im->N,
+                      s));
     if (timed && uses_status(im, NV))
         CK(cudaMemcpyAsync(im->h_status, im->d_status, sizeof(int), cudaMemcpyDeviceToHost, s));
     if (timed) CK(cudaEventRecord(e[6], s));

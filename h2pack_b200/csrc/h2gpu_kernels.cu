@@ -777,18 +777,35 @@ __global__ void __launch_bounds__(kThreads) k_down(const DownTask* __restrict__ 
     }
 }
 
+// Sum of one element over n slots, in slot order, eight loads in flight.
+__device__ __forceinline__ double slot_sum(const double* __restrict__ p, const int* __restrict__ sl, int n, int NV)
+{
+    double s = 0.0;
+    int k = 0;
+    for (; k + 8 <= n; k += 8)
+    {
+        double a[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) a[u] = p[(long long) sl[k + u] * NV];
+#pragma unroll
+        for (int u = 0; u < 8; u++) s += a[u];
+    }
+    for (; k < n; k++) s += p[(long long) sl[k] * NV];
+    return s;
+}
+
+// The slot sums are bound by HBM (each slot row is read once); what kept them from it was
+// one CTA per node walking its elements one after the other, each a chain of dependent
+// load / add steps.  The elements of a node are spread over gridDim.y CTAs
+// (sum_grid_y) and slot_sum keeps eight loads in flight.
 // y1 of a node = sum of its PS slots (fixed order); rows indexed like the y0 region.
 template <int NV>
 __global__ void k_y1sum(const Y1Task* __restrict__ tasks, const int* __restrict__ slots,
                         const double* __restrict__ PS, double* __restrict__ Y1)
 {
     const Y1Task t = tasks[blockIdx.x];
-    for (int i = threadIdx.x; i < t.nrow * NV; i += blockDim.x)
-    {
-        double s = 0.0;
-        for (int k = t.slot_beg; k < t.slot_end; k++) s += PS[(long long) slots[k] * NV + i];
-        Y1[(long long) t.row * NV + i] = s;
-    }
+    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < t.nrow * NV; i += blockDim.x * gridDim.y)
+        Y1[(long long) t.row * NV + i] = slot_sum(PS + i, slots + t.slot_beg, t.slot_end - t.slot_beg, NV);
 }
 
 // --------------------------------------------------------------- assemble
@@ -800,13 +817,12 @@ __global__ void k_asm(const AsmTask* __restrict__ tasks, const int* __restrict__
                       double* __restrict__ Y, long long y_rs, long long y_cs, int nv)
 {
     const AsmTask t = tasks[blockIdx.x];
-    for (int i = threadIdx.x; i < t.nrow * NV; i += blockDim.x)
+    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < t.nrow * NV; i += blockDim.x * gridDim.y)
     {
         int r = i / NV, v = i % NV;
         if (v >= nv) continue;
-        double s = 0.0;
-        for (int k = t.slot_beg; k < t.slot_end; k++) s += PS[(long long) (slots[k] + r) * NV + v];
-        Y[(long long) fwd[t.row0 + r] * y_rs + (long long) v * y_cs] = s;
+        Y[(long long) fwd[t.row0 + r] * y_rs + (long long) v * y_cs] =
+            slot_sum(PS + i, slots + t.slot_beg, t.slot_end - t.slot_beg, NV);
     }
 }
 
@@ -3722,18 +3738,29 @@ cudaError_t launch_down(int NV, const DownTask* t, int n, const TA* U, const dou
     return cudaGetLastError();
 }
 
-cudaError_t launch_y1sum(int NV, const Y1Task* t, int n, const int* slots, const double* PS, double* Y1, cudaStream_t st)
+// CTAs per task of the slot sums: one element per thread for an average task, as long as
+// that stays within 32 CTAs per SM in all (beyond it the launch is HBM-bound anyway).
+static int sum_grid_y(int n, long long rows, int NV)
+{
+    const long long per = (rows * NV / n + 255) / 256, most = (148 * 32 + n - 1) / n;
+    return (int) (per < 1 ? 1 : per < most ? per : most);
+}
+
+cudaError_t launch_y1sum(int NV, const Y1Task* t, int n, const int* slots, const double* PS, double* Y1, long long rows,
+                         cudaStream_t st)
 {
     if (n <= 0) return cudaSuccess;
-    NV_DISPATCH_WIDE(NV, k_y1sum<NVc><<<n, 256, 0, st>>>(t, slots, PS, Y1));
+    const dim3 g(n, sum_grid_y(n, rows, NV));
+    NV_DISPATCH_WIDE(NV, k_y1sum<NVc><<<g, 256, 0, st>>>(t, slots, PS, Y1));
     return cudaGetLastError();
 }
 
 cudaError_t launch_asm(int NV, const AsmTask* t, int n, const int* slots, const double* PS, const int* fwd,
-                       double* Y, long long y_rs, long long y_cs, int nv, cudaStream_t st)
+                       double* Y, long long y_rs, long long y_cs, int nv, long long rows, cudaStream_t st)
 {
     if (n <= 0) return cudaSuccess;
-    NV_DISPATCH_WIDE(NV, k_asm<NVc><<<n, 256, 0, st>>>(t, slots, PS, fwd, Y, y_rs, y_cs, nv));
+    const dim3 g(n, sum_grid_y(n, rows, NV));
+    NV_DISPATCH_WIDE(NV, k_asm<NVc><<<g, 256, 0, st>>>(t, slots, PS, fwd, Y, y_rs, y_cs, nv));
     return cudaGetLastError();
 }
 

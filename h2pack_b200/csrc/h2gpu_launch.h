@@ -29,9 +29,11 @@ cudaError_t launch_split3(const double* XS, long long row0, long long n, long lo
 template <typename TA>
 cudaError_t launch_down(int NV, const DownTask* t, int n, const TA* U, const double* Y1, double* PS, double* PUSH,
                         cudaStream_t st, int use_tc = 0);
-cudaError_t launch_y1sum(int NV, const Y1Task* t, int n, const int* slots, const double* PS, double* Y1, cudaStream_t st);
+// rows: rows of all the tasks together (the grid's size follows from it)
+cudaError_t launch_y1sum(int NV, const Y1Task* t, int n, const int* slots, const double* PS, double* Y1, long long rows,
+                         cudaStream_t st);
 cudaError_t launch_asm(int NV, const AsmTask* t, int n, const int* slots, const double* PS, const int* fwd,
-                       double* Y, long long y_rs, long long y_cs, int nv, cudaStream_t st);
+                       double* Y, long long y_rs, long long y_cs, int nv, long long rows, cudaStream_t st);
 // far: every source set is admissible for its target (r > 0); ppts / pin / tiles: the
 // source panels and tile lists, which the tensor-core kernel (FP32 scalar kernels,
 // NV 8 / 16, use_tc) reads; lo / plo: the low parts of the FP32 points and of the
