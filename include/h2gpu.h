@@ -422,9 +422,10 @@ int h2gpu_pp_sketch_id(int kernel_id, const double *krnl_param, int n_krnl_param
  *   L[i], l_ld[i]       ULV_L[i]: m[i] x m[i] row-major;
  *   p[i]                LU only: ULV_p[i], m[i] - Ls[i] entries.
  * The device keeps each node's explicit Q (formed from the reflectors at create) and
- * L, both m x m, and runs one launch per tree level per sweep (one CTA per node, the
- * node's vector in shared memory: nodes of more than 13,872 rows are refused with
- * H2GPU_ERR_UNSUPPORTED).
+ * L, both m x m, with the inverses of the triangular factor's 64 x 64 diagonal blocks, and
+ * runs one launch per tree level per sweep (units of 64 rows over the whole GPU, which
+ * wait for one another through bounded waits: H2GPU_ERR_DEVICE from the next call if one
+ * expires; nodes of more than 13,872 rows are refused with H2GPU_ERR_UNSUPPORTED).
  */
 typedef struct h2gpu_ulv h2gpu_ulv;
 
