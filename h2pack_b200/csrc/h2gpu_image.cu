@@ -930,7 +930,8 @@ int build_plan(h2gpu_image* im, const h2gpu_desc* d, HostPlan& hp)
                         for (int j0 = 0; j0 < js[k].npt; j0 += 128)
                         {
                             const int nj = std::min(128, js[k].npt - j0);
-                            hp.tiles.push_back(TileRec{js[k].grp + j0 / 8, (nj + 7) / 8, nj, 0, js[k].sx, js[k].sy, js[k].sz, 0.f});
+                            hp.tiles.push_back(TileRec{js[k].grp + j0 / 8, (nj + 7) / 8, nj, js[k].pt0 + j0, js[k].sx, js[k].sy, js[k].sz,
+                                                       js[k].in_row + kd * j0});
                         }
                     ins.first->second.second = (int) hp.tiles.size();
                     REQ(hp.tiles.size() < (1u << 30), "too many source tiles");
@@ -1532,7 +1533,8 @@ int check_plan(const h2gpu_image* im, const h2gpu_desc* d, const HostPlan& hp, l
                         REQ(k < t.tile_end && k < (int) hp.tiles.size(), "plan: a target has too few source tiles");
                         const TileRec& T = hp.tiles[k];
                         const int nj = std::min(128, hp.js[si].npt - j0);
-                        REQ(T.nj == nj && T.ng == (nj + 7) / 8 && T.gb == hp.js[si].grp + j0 / 8,
+                        REQ(T.nj == nj && T.ng == (nj + 7) / 8 && T.gb == hp.js[si].grp + j0 / 8 &&
+                                T.pt0 == hp.js[si].pt0 + j0 && T.in_row == hp.js[si].in_row + kd * j0,
                             "plan: source tiles do not cover a source set in order");
                     }
                 REQ(k == t.tile_end, "plan: a target has too many source tiles");

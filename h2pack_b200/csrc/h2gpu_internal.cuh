@@ -95,7 +95,7 @@ struct JitTarget {
     int out_row;       // row of the chunk's first output row (PS, or Y1 when out_y1)
     int out_y1;        // 1: outputs are the node's y1 rows
     int src_beg, src_end;
-    int tile_beg, tile_end;   // its source tiles (FP32 tensor-core path)
+    int tile_beg, tile_end;   // its source tiles
 };
 
 struct JitSource {
@@ -109,15 +109,15 @@ struct JitSource {
 // points, padded at its end.  Per group, the points in the pairs the m16n8k8 B fragment
 // holds them (static) and the inputs split into TF32 hi / lo in A-fragment order
 // (refilled from XS for every panel of right-hand sides).
-// One tile (up to 128 points) of a source set for a target (FP32 tensor-core JIT path):
-// the tiles of all the target's source sets in order, so the kernel walks one array.
+// One tile (up to 128 points) of a source set for a target: the tiles of all the target's
+// source sets in order, so the kernels (FP32 on the tensor cores, FP64) walk one array.
 struct TileRec {
     int gb;            // first panel group of the tile
     int ng;            // groups in the tile (1..16)
     int nj;            // points in the tile (1..128)
-    int pad0;
+    int pt0;           // point-space index of its first point
     float sx, sy, sz;  // center(target set) - center(source set)
-    float pad1;
+    int in_row;        // XS row of the input of its first point
 };
 
 struct PanelGroup {

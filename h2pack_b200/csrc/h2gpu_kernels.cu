@@ -15,6 +15,7 @@
 // reproducible run to run.
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
+#include <cooperative_groups.h>
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
@@ -1114,6 +1115,356 @@ __global__ void __launch_bounds__(128 / TPT, sizeof(T) == 4 ? 5 * TPT : 4 * TPT)
             else o[k] = (double) acc[q][k];
         }
     }
+}
+
+// ---------------------------------------------------------- JIT owner kernel, FP64
+//
+// FP64 kernel evaluation.  The FP64 pipe bounds the FP64 path, so the values are formed with
+// as few FP64 operations as a result within about one unit in the last place takes; every
+// argument outside the fast path's range (zero or denormal or non-finite r^2, |t| >= 700)
+// goes to the CUDA math functions of Scalar<KID, double>.
+
+// 1 / sqrt(x) for normal x: the hardware approximation and one step of Householder's
+// third-order iteration, y (1 + e/2 + 3 e^2/8) with e = 1 - x y^2 (|e| < 2^-19)
+__device__ __forceinline__ double rsqrt_seed(double x)
+{
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    return y;
+}
+__device__ __forceinline__ double rsqrt64(double x)
+{
+    const double y = rsqrt_seed(x), e = fma(-(x * y), y, 1.0);
+    return fma(fma(0.375, e, 0.5), y * e, y);
+}
+// sqrt(x) for normal x: Goldschmidt's coupled iteration for sqrt(x) and 1 / (2 sqrt(x)),
+// then one correction with the residual x - g^2
+__device__ __forceinline__ double sqrt64(double x)
+{
+    const double y = rsqrt_seed(x);
+    double g = x * y, h = 0.5 * y;
+    const double r = fma(-g, h, 0.5);
+    g = fma(g, r, g);
+    h = fma(h, r, h);
+    return fma(fma(-g, g, x), h, g);
+}
+// exp(t), |t| < 700: table-driven (P. T. P. Tang, ACM TOMS 15(2), 1989) with 16 entries,
+// t = (16 m + j) ln2/16 + r, exp(t) = 2^m 2^(j/16) (1 + p(r)), |r| <= ln2/32; p is the
+// minimax polynomial of degree 6 with p'(0) = 1 (error 1.2e-17).  Sixteen doubles are one
+// row of the shared-memory banks: any lanes' reads are free of conflicts.
+__device__ const double kExp2Sixteenth[16] = {
+    0x1.0000000000000p+0, 0x1.0b5586cf9890fp+0, 0x1.172b83c7d517bp+0, 0x1.2387a6e756238p+0,
+    0x1.306fe0a31b715p+0, 0x1.3dea64c123422p+0, 0x1.4bfdad5362a27p+0, 0x1.5ab07dd485429p+0,
+    0x1.6a09e667f3bcdp+0, 0x1.7a11473eb0187p+0, 0x1.8ace5422aa0dbp+0, 0x1.9c49182a3f090p+0,
+    0x1.ae89f995ad3adp+0, 0x1.c199bdd85529cp+0, 0x1.d5818dcfba487p+0, 0x1.ea4afa2a490dap+0};
+__device__ __forceinline__ double exp64(double t, const double* tab)
+{
+    const double shift = 6755399441055744.0;                  // 1.5 2^52: the sum's low word is the integer
+    double n = fma(t, 0x1.71547652b82fep+4, shift);           // 16 / ln 2
+    const int k = __double2loint(n);
+    n -= shift;
+    double r = fma(n, -0x1.62e42f8000000p-5, t);              // ln2 / 16 in two parts, the first of 26 bits
+    r = fma(n, -0x1.be8e7bcd5e4f2p-31, r);
+    double q = fma(r, 0x1.6c185df9f6f0cp-10, 0x1.11123abf01f8ep-7);
+    q = fma(r, q, 0x1.555555545e9c7p-5);
+    q = fma(r, q, 0x1.555555548f728p-3);
+    q = fma(r, q, 0x1.0000000000005p-1);
+    const double p = fma(r * r, q, r);
+    double s = tab[k & 15];
+    s = __hiloint2double(__double2hiint(s) + ((k >> 4) << 20), __double2loint(s));
+    return fma(s, p, s);
+}
+// The fast forms and their range of r^2: the high word of r^2 less lo, as an unsigned number,
+// is below span (which excludes what the fast form does not take: zero and denormal r^2,
+// |t| >= 700, infinities and NaN).  They are free of branches, so that a lane's values are
+// evaluated side by side; values out of range are made again by slow().
+struct Range64 {
+    unsigned lo, span;
+    __device__ __forceinline__ bool has(double r2) const { return (unsigned) __double2hiint(r2) - lo < span; }
+};
+__device__ __forceinline__ unsigned high_word(double x) { return (unsigned) __double2hiint(x); }
+template <int KID> struct Fast64;
+template <> struct Fast64<KRNL_COULOMB_ID> {
+    static __device__ __forceinline__ Range64 range(double, double) { return Range64{0x00100000u, 0x7fe00000u}; }
+    static __device__ __forceinline__ double f(double r2, double, double, const double*) { return rsqrt64(r2); }
+};
+template <> struct Fast64<KRNL_GAUSSIAN_ID> {
+    static __device__ __forceinline__ Range64 range(double p0, double)
+    {
+        return Range64{0u, high_word(fmin(700.0 / fabs(p0), 1e300))};
+    }
+    static __device__ __forceinline__ double f(double r2, double p0, double, const double* tab) { return exp64(-p0 * r2, tab); }
+};
+template <> struct Fast64<KRNL_MATERN32_ID> {
+    static __device__ __forceinline__ Range64 range(double, double c0)
+    {
+        const unsigned top = high_word(fmin(490000.0 / (c0 * c0), 1e300));
+        return Range64{0x00100000u, top > 0x00100000u ? top - 0x00100000u : 0u};
+    }
+    static __device__ __forceinline__ double f(double r2, double, double c0, const double* tab)
+    {
+        const double t = c0 * sqrt64(r2), e = exp64(t, tab);
+        return fma(-t, e, e);
+    }
+};
+
+// rpy_coef<double> for spheres apart (r > ta + sa), with 1 / r by rsqrt64 and the products
+// arranged for few operations
+__device__ __forceinline__ void rpy_far64(double dx, double dy, double dz, double r2, double ta, double sa, double C,
+                                          double& t1, double& t2, double& ux, double& uy, double& uz)
+{
+    const double inv = rsqrt64(r2);
+    ux = dx * inv; uy = dy * inv; uz = dz * inv;
+    const double a = C * 0.75 * inv, b = fma(ta, ta, sa * sa) * (inv * inv);
+    t1 = fma(a * b, 1.0 / 3.0, a);
+    t2 = fma(-a, b, a);
+}
+
+// d += a b of 8 x 4 and 4 x 8 FP64 values: a: (row lane / 4, column lane % 4), b: (row lane % 4,
+// column lane / 4), d: (row lane / 4, columns 2 (lane % 4) and the next)
+__device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b)
+{
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};" : "+d"(d[0]), "+d"(d[1]) : "d"(a), "d"(b));
+}
+
+// A chunk of <= 128 target points and a share of its source tiles per CTA, four CTAs per SM.
+// What bounds it: the FP64 pipe (a kernel value takes 14 to 25 operations, each right-hand
+// side one more, in DMMA as in DFMA: 17 and 18 T multiply-adds/s measured, not in
+// addition).  A warp walks 32 targets, four sources at a time: a lane evaluates source
+// lane % 4 against the targets lane / 4 + 8 g, so the four values are independent chains and
+// one read of a source and its inputs serves all four (with one target per thread the
+// broadcast reads of 16 inputs per value bound the kernel: 128 bytes per lane for 16
+// operations).  Two steps of the sources at once (unroll 2), or half the warps with twice the
+// registers, measured the same or slower.  Before -> now, one B200: Matern N = 120,000, 16
+// right-hand sides: far field 14.2 -> 9.6 ms, near 3.2 -> 2.1; one right-hand side, N =
+// 100,000: 11.7 -> 5.2 and 2.1 -> 1.3; Coulomb N = 30,011, 3: 2.0 -> 0.56 and 0.31 -> 0.10;
+// Gaussian N = 10,007, 1: 0.39 -> 0.14 and 0.33 -> 0.09.  Panels of 8 and 16 scalar right-hand sides: the value is the lane's entry of
+// a DMMA's A fragment; others: multiply-adds into the lane's own sums, added over lane % 4
+// at the end.  Warps that a chunk leaves over (<= 64 or <= 32 targets) take every 2nd or
+// 4th step of the sources.  Small images have fewer chunks than the GPU has CTA slots:
+// there the CTAs of a cluster share a chunk, each taking every S-th source tile, and their
+// sums meet in the first CTA through distributed shared memory, in rank order.  Outputs are
+// written once, no atomics.
+template <int NV, int KD> struct Jit64Cfg {
+    static constexpr int W = KD * NV;
+    static constexpr bool MMA = KD == 1 && NV >= 8;
+    static constexpr int G = KD == 1 || NV == 1 ? 4 : NV == 2 ? 2 : 1;   // targets per lane
+    static constexpr int TILE = W > 8 ? 64 : 128;                       // sources staged at a time
+    // row stride of the staged inputs: DMMA fragments read four rows of eight at once
+    static constexpr int LD = MMA ? W + 4 : W;
+    static constexpr int BUF = TILE * LD > 128 * W ? TILE * LD : 128 * W;   // inputs, then the warps' sums
+    static constexpr int NT = 32 * (128 / (8 * G));                     // threads: a warp per 8 G targets
+    // warps per SM: 16 of 128 registers; four RPY values at once take 168 (3.5 -> 0.98 ms for N =
+    // 20,011, one right-hand side; 1.03 ms with 128 and spills)
+    static constexpr int CTAS = (KD == 3 && G == 4 ? 384 : 512) / NT;
+};
+template <int KID, int NV, int KD>
+__global__ void __launch_bounds__(Jit64Cfg<NV, KD>::NT, Jit64Cfg<NV, KD>::CTAS)
+    k_jit64(const JitTarget* __restrict__ tgts, const TileRec* __restrict__ tiles, const double4* __restrict__ pts,
+            KParam kp, const double* __restrict__ XS, double* __restrict__ PS, double* __restrict__ Y1, int S)
+{
+    namespace cg = cooperative_groups;
+    using C = Jit64Cfg<NV, KD>;
+    constexpr int W = C::W, G = C::G, TILE = C::TILE, LD = C::LD, NT = C::NT, WT = 8 * G, NWARP = NT / 32;
+    __shared__ __align__(16) double s_tab[16];
+    __shared__ __align__(16) double4 s_pt[TILE];
+    __shared__ __align__(16) double s_buf[C::BUF];
+    const int rank = (int) (blockIdx.x & (S - 1));
+    const JitTarget tg = tgts[blockIdx.x / S];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, q = lane & 3, row = lane >> 2;
+    // warps with targets, shares of the sources, this warp's targets and how many groups of 8
+    const int nw = (tg.npt + WT - 1) / WT, ns = NWARP / nw;
+    const int wt = warp % nw, share = warp / nw;
+    const int groups = share < ns ? (min(WT, tg.npt - WT * wt) + 7) >> 3 : 0;
+    if (tid < 16) s_tab[tid] = kExp2Sixteenth[tid];
+    double xi[G], yi[G], zi[G], ri[KD == 3 ? G : 1];
+#pragma unroll
+    for (int g = 0; g < G; g++)
+    {
+        const double4 x = pts[tg.pt0 + min(WT * wt + 8 * g + row, tg.npt - 1)];
+        xi[g] = x.x; yi[g] = x.y; zi[g] = x.z;
+        if constexpr (KD == 3) ri[g] = x.w;
+    }
+    const double p0 = kp.p0, c0 = kp.c0;
+    constexpr int NA = C::MMA ? NV / 8 : W;         // accumulators per target group: C fragments, or sums
+    double acc[G][NA][C::MMA ? 2 : 1];
+#pragma unroll
+    for (int g = 0; g < G; g++)
+#pragma unroll
+        for (int k = 0; k < NA; k++)
+#pragma unroll
+            for (int h = 0; h < (C::MMA ? 2 : 1); h++) acc[g][k][h] = 0.0;
+    // the values of one source against the lane's G targets
+    [[maybe_unused]] Range64 range{};
+    if constexpr (KD == 1) range = Fast64<KID>::range(p0, c0);
+    [[maybe_unused]] auto values = [&](const double4& pj, double (&k)[G]) {
+        if constexpr (KD == 1)
+        {
+            double r2[G];
+            bool slow = false;
+#pragma unroll
+            for (int g = 0; g < G; g++)
+            {
+                const double dx = xi[g] - pj.x, dy = yi[g] - pj.y, dz = zi[g] - pj.z;
+                r2[g] = fma(dz, dz, fma(dy, dy, dx * dx));
+                k[g] = Fast64<KID>::f(r2[g], p0, c0, s_tab);
+                slow |= !range.has(r2[g]);
+            }
+            if (slow)
+#pragma unroll 1
+                for (int g = 0; g < G; g++)
+                {
+                    double x = r2[0];
+#pragma unroll
+                    for (int h = 1; h < G; h++) x = h == g ? r2[h] : x;
+                    if (range.has(x)) continue;
+                    x = Scalar<KID, double>::f(x, p0, c0);
+#pragma unroll
+                    for (int h = 0; h < G; h++) k[h] = h == g ? x : k[h];
+                }
+        }
+    };
+    for (int t = tg.tile_beg + rank; t < tg.tile_end; t += S)
+    {
+        const TileRec R = tiles[t];
+        for (int j0 = 0; j0 < R.nj; j0 += TILE)
+        {
+            const int nj = min(TILE, R.nj - j0), n4 = (nj + 3) & ~3;
+            __syncthreads();
+            // sources past the end: the last point again, with zero inputs
+            for (int j = tid; j < n4; j += NT) s_pt[j] = pts[R.pt0 + j0 + min(j, nj - 1)];
+            const double* src = XS + (long long) (R.in_row + KD * j0) * NV;
+            if constexpr (W % 2 == 0)
+            {
+                constexpr int H = W / 2;
+                for (int e = tid; e < n4 * H; e += NT)
+                    *reinterpret_cast<double2*>(s_buf + (e / H) * LD + 2 * (e % H)) =
+                        e < nj * H ? *reinterpret_cast<const double2*>(src + 2 * e) : make_double2(0.0, 0.0);
+            } else {
+                for (int e = tid; e < n4 * W; e += NT) s_buf[e] = e < nj * W ? src[e] : 0.0;
+            }
+            __syncthreads();
+            if (groups == 0) continue;
+            for (int j = 4 * share + q; j < n4; j += 4 * ns)
+            {
+                const double4 pj = s_pt[j];
+                if constexpr (C::MMA)
+                {
+                    double b[NA];
+#pragma unroll
+                    for (int k = 0; k < NA; k++) b[k] = s_buf[j * LD + row + 8 * k];
+                    double k[G];
+                    values(pj, k);
+#pragma unroll
+                    for (int g = 0; g < G; g++)
+                    {
+                        if (j >= nj) k[g] = 0.0;
+                        if (g < groups)
+#pragma unroll
+                            for (int v = 0; v < NA; v++) mma_f64(acc[g][v], k[g], b[v]);
+                    }
+                } else {
+                    double in[W];
+#pragma unroll
+                    for (int k = 0; k < W; k++) in[k] = s_buf[j * LD + k];   // zeros past the end
+                    if constexpr (KD == 1)
+                    {
+                        double k[G];
+                        values(pj, k);
+#pragma unroll
+                        for (int g = 0; g < G; g++)
+                        {
+                            if (j >= nj) k[g] = 0.0;
+#pragma unroll
+                            for (int v = 0; v < NV; v++) acc[g][v][0] = fma(k[g], in[v], acc[g][v][0]);
+                        }
+                    } else {
+                        double t1[G], t2[G], ux[G], uy[G], uz[G];
+                        bool slow = false;
+#pragma unroll
+                        for (int g = 0; g < G; g++)
+                        {
+                            const double dx = xi[g] - pj.x, dy = yi[g] - pj.y, dz = zi[g] - pj.z, ab = ri[g] + pj.w;
+                            const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
+                            rpy_far64(dx, dy, dz, r2, ri[g], pj.w, c0, t1[g], t2[g], ux[g], uy[g], uz[g]);
+                            slow |= !(r2 > ab * ab && high_word(r2) - 0x00100000u < 0x7fe00000u);
+                        }
+                        if (slow)
+#pragma unroll 1
+                            for (int g = 0; g < G; g++)
+                            {
+                                const double dx = xi[g] - pj.x, dy = yi[g] - pj.y, dz = zi[g] - pj.z;
+                                double c[5];
+                                rpy_coef<double>(dx, dy, dz, ri[g], pj.w, c0, c[0], c[1], c[2], c[3], c[4]);
+#pragma unroll
+                                for (int h = 0; h < G; h++)
+                                    if (h == g) { t1[h] = c[0]; t2[h] = c[1]; ux[h] = c[2]; uy[h] = c[3]; uz[h] = c[4]; }
+                            }
+#pragma unroll
+                        for (int g = 0; g < G; g++)
+                        {
+                            if (j >= nj) { t1[g] = 0.0; t2[g] = 0.0; ux[g] = 0.0; uy[g] = 0.0; uz[g] = 0.0; }
+#pragma unroll
+                            for (int v = 0; v < NV; v++)
+                            {
+                                const double bx = in[v], by = in[NV + v], bz = in[2 * NV + v];
+                                const double dot = t2[g] * fma(uz[g], bz, fma(uy[g], by, ux[g] * bx));
+                                acc[g][v][0] = fma(dot, ux[g], fma(t1[g], bx, acc[g][v][0]));
+                                acc[g][NV + v][0] = fma(dot, uy[g], fma(t1[g], by, acc[g][NV + v][0]));
+                                acc[g][2 * NV + v][0] = fma(dot, uz[g], fma(t1[g], bz, acc[g][2 * NV + v][0]));
+                            }
+                        }
+                    }
+                }
+            }
+            __syncwarp();
+        }
+    }
+    // every warp's sums to shared memory, [target][right-hand side]; then the sum over the
+    // shares and the cluster's CTAs
+    __syncthreads();
+    double* const o = s_buf + warp * WT * W;
+    if (groups > 0)
+#pragma unroll
+        for (int g = 0; g < G; g++)
+        {
+            double* const og = o + (8 * g + row) * W;
+            if constexpr (C::MMA)
+            {
+#pragma unroll
+                for (int k = 0; k < NA; k++)
+                {
+                    og[8 * k + 2 * q] = acc[g][k][0];
+                    og[8 * k + 2 * q + 1] = acc[g][k][1];
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < W; k++)
+                {
+                    double s = acc[g][k][0];
+                    s += __shfl_xor_sync(kFull, s, 1);
+                    s += __shfl_xor_sync(kFull, s, 2);
+                    if (q == 0) og[k] = s;
+                }
+            }
+        }
+    __syncthreads();
+    if (S > 1) cg::this_cluster().sync();
+    if (rank == 0)
+    {
+        double* const out = (tg.out_y1 ? Y1 : PS) + (long long) tg.out_row * NV;
+        for (int e = tid; e < tg.npt * W; e += NT)
+        {
+            double s = 0.0;
+            for (int r = 0; r < S; r++)
+            {
+                const double* b = S > 1 ? cg::this_cluster().map_shared_rank(s_buf, r) : s_buf;
+                for (int g = 0; g < ns; g++) s += b[g * nw * WT * W + e];
+            }
+            out[e] = s;
+        }
+    }
+    if (S > 1) cg::this_cluster().sync();      // shared memory stays until it has been read
 }
 
 // FP32 scalar kernels on the CUDA cores (the panels the tensor-core kernel does not
@@ -3764,6 +4115,35 @@ cudaError_t launch_asm(int NV, const AsmTask* t, int n, const int* slots, const 
     return cudaGetLastError();
 }
 
+// CTAs per target chunk (the CTAs of a cluster share a chunk's source tiles): the smallest
+// power of two that gives the launch two waves of the SMs' CTA slots, at most 8 (the portable
+// cluster size).
+static int jit_split(int n, int per_sm)
+{
+    int S = 1;
+    while (S < 8 && (long long) n * S < 2LL * 148 * per_sm) S *= 2;
+    return S;
+}
+
+// n * S CTAs in clusters of S
+template <typename... P, typename... A>
+static cudaError_t launch_cluster(void (*kern)(P...), int n, int S, int threads, int smem, cudaStream_t st, A... args)
+{
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3((unsigned) n * S);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    cudaLaunchAttribute a[1];
+    a[0].id = cudaLaunchAttributeClusterDimension;
+    a[0].val.clusterDim.x = S;
+    a[0].val.clusterDim.y = 1;
+    a[0].val.clusterDim.z = 1;
+    c.attrs = a;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kern, (P) args...);
+}
+
 template <int KID, typename T, int KD>
 static cudaError_t launch_jit_k(int NV, const JitTarget* tg, int n, const JitSource* sr, const void* pts, KParam kp,
                                 int use_shift, int use_tc, const double* XS, double* PS, double* Y1, cudaStream_t st,
@@ -3796,11 +4176,17 @@ static cudaError_t launch_jit_k(int NV, const JitTarget* tg, int n, const JitSou
         }
     }
     // FP32: two targets per thread (64 threads per 128-point chunk) where the accumulators
-    // allow it; FP64: one target per thread, 4 CTAs per SM (two targets per thread took
-    // 188 registers and left 7 warps per SM to hide the FP64 latencies: 1.4x slower)
+    // allow it; FP64: one target per thread (two took 188 registers and left 7 warps per SM
+    // to hide the FP64 latencies: 1.4x slower)
     NV_DISPATCH(NV, {
         if constexpr (KD == 3 && NVc > 8)
             return cudaErrorInvalidValue;   // tensor kernels run in panels of <= 8 right-hand sides
+        else if constexpr (sizeof(T) == 8)
+        {
+            if (!tiles) return cudaErrorInvalidValue;
+            const int S = jit_split(n, 4);
+            return launch_cluster(k_jit64<KID, NVc, KD>, n, S, Jit64Cfg<NVc, KD>::NT, 0, st, tg, tiles, p, kp, XS, PS, Y1, S);
+        }
         else if constexpr (KD == 1 && sizeof(T) == 4)
         {
             // scalar FP32 kernels: the two targets of a thread as one FP32x2 pair
