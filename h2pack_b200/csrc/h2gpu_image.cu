@@ -115,7 +115,6 @@ struct h2gpu_image {
     int n_wide[4] = {0, 0, 0, 0};
     JitTarget* d_jtN = nullptr;
     JitTarget* d_jtF = nullptr;
-    JitSource* d_js = nullptr;
     AsmTask* d_asm = nullptr;
     int* d_asm_slots = nullptr;
     int* d_fwd = nullptr;
@@ -199,7 +198,7 @@ namespace {
 void free_all(h2gpu_image* im)
 {
     void* ptrs[] = {im->d_up, im->d_dn, im->d_y1t, im->d_y1_slots, im->d_blkB, im->d_blkD, im->d_jtN, im->d_jtF,
-                    im->d_js, im->d_asm, im->d_asm_slots, im->d_fwd, im->d_bwd, im->d_U64, im->d_U32, im->d_B64,
+                    im->d_asm, im->d_asm_slots, im->d_fwd, im->d_bwd, im->d_U64, im->d_U32, im->d_B64,
                     im->d_B32, im->d_D64, im->d_D32, im->d_pts64, im->d_pts32, im->d_XS, im->d_PS, im->d_Y1,
                     im->d_PUSH, im->d_io, im->d_owN, im->d_owF, im->d_pp, im->d_jtN2, im->d_jtF2, im->d_y1t2,
                     im->d_y1_slots2, im->d_asm2, im->d_asm_slots2, im->d_status, im->d_pg, im->d_ppts,
@@ -1631,7 +1630,6 @@ int upload_plan(h2gpu_image* im, const h2gpu_desc* d, HostPlan& hp)
     TRY(upload(hp.wide, &im->d_wide, im->bytes));
     TRY(upload(hp.jtN, &im->d_jtN, im->bytes));
     TRY(upload(hp.jtF, &im->d_jtF, im->bytes));
-    TRY(upload(hp.js, &im->d_js, im->bytes));
     TRY(upload(hp.at, &im->d_asm, im->bytes));
     TRY(upload(hp.at_slots, &im->d_asm_slots, im->bytes));
     TRY(upload(hp.fw, &im->d_fwd, im->bytes));
@@ -1819,7 +1817,7 @@ int run_panel(h2gpu_image* im, int NV, int nv, const double* X, long long x_rs, 
         CK(launch_gather(NV, X, x_rs, x_cs, nv, im->d_fwd, im->N, im->d_XS, s));
         if (timed) CK(cudaEventRecord(e[1], s));
         CK(launch_panel_in(NV, im->d_pg, 0, im->n_pg_pts, im->d_XS, im->d_pin, s));
-        CK(launch_jit(im->kernel_id, 1, NV, im->d_jtN2, im->n_jtN2, im->d_js, im->d_pts32, kp, 1, 1, im->d_XS,
+        CK(launch_jit(im->kernel_id, 1, NV, im->d_jtN2, im->n_jtN2, im->d_pts32, kp, 1, 1, im->d_XS,
                       im->d_PS, im->d_Y1, s, 0, im->d_ppts, im->d_pin, im->d_tiles, im->d_pts32lo, im->d_pplo));
         CK(launch_pair(im->kernel_id, NV, im->d_owN, im->n_owN, im->d_pp, im->d_pts32, kp, im->d_XS, im->d_PS, s, 0,
                        im->d_pts32lo));
@@ -1833,7 +1831,7 @@ int run_panel(h2gpu_image* im, int NV, int nv, const double* X, long long x_rs, 
         CK(launch_pair(im->kernel_id, NV, im->d_owF, im->n_owF, im->d_pp, im->d_pts32, kp, im->d_XS, im->d_PS, s,
                        im->far_diff ? 0 : 1, im->d_pts32lo));
         CK(launch_panel_in(NV, im->d_pg, im->n_pg_pts, im->n_pg - im->n_pg_pts, im->d_XS, im->d_pin, s));
-        CK(launch_jit(im->kernel_id, 1, NV, im->d_jtF2, im->n_jtF2, im->d_js, im->d_pts32, kp, 1, 1, im->d_XS,
+        CK(launch_jit(im->kernel_id, 1, NV, im->d_jtF2, im->n_jtF2, im->d_pts32, kp, 1, 1, im->d_XS,
                       im->d_PS, im->d_Y1, s, im->far_diff ? 0 : 1, im->d_ppts, im->d_pin, im->d_tiles, im->d_pts32lo,
                       im->d_pplo));
         CK(launch_y1sum(NV, im->d_y1t2, im->n_y12, im->d_y1_slots2, im->d_PS, im->d_Y1, im->y0_rows, s));
@@ -1875,7 +1873,7 @@ int run_panel(h2gpu_image* im, int NV, int nv, const double* X, long long x_rs, 
     } else {
         const bool panels = f32 && panels_used(im, NV);
         if (panels) CK(launch_panel_in(NV, im->d_pg, 0, im->n_pg_pts, im->d_XS, im->d_pin, s));
-        CK(launch_jit(im->kernel_id, f32, NV, im->d_jtN, im->n_jtN, im->d_js, f32 ? (const void*) im->d_pts32 : (const void*) im->d_pts64,
+        CK(launch_jit(im->kernel_id, f32, NV, im->d_jtN, im->n_jtN, f32 ? (const void*) im->d_pts32 : (const void*) im->d_pts64,
                       kparam_of(im), f32 ? 1 : 0, im->jit_tc, im->d_XS, im->d_PS, im->d_Y1, s, 0, im->d_ppts, im->d_pin, im->d_tiles,
                       im->d_pts32lo, im->d_pplo));
         im->st.n_launches += panels ? 1 : 0;
@@ -1908,7 +1906,7 @@ int run_panel(h2gpu_image* im, int NV, int nv, const double* X, long long x_rs, 
     } else {
         const bool panels = f32 && panels_used(im, NV);
         if (panels) CK(launch_panel_in(NV, im->d_pg, im->n_pg_pts, im->n_pg - im->n_pg_pts, im->d_XS, im->d_pin, s));
-        CK(launch_jit(im->kernel_id, f32, NV, im->d_jtF, im->n_jtF, im->d_js, f32 ? (const void*) im->d_pts32 : (const void*) im->d_pts64,
+        CK(launch_jit(im->kernel_id, f32, NV, im->d_jtF, im->n_jtF, f32 ? (const void*) im->d_pts32 : (const void*) im->d_pts64,
                       kparam_of(im), f32 ? 1 : 0, im->jit_tc, im->d_XS, im->d_PS, im->d_Y1, s, im->far_diff ? 0 : 1,
                       im->d_ppts, im->d_pin, im->d_tiles, im->d_pts32lo, im->d_pplo));
         im->st.n_launches += panels ? 1 : 0;

@@ -992,6 +992,25 @@ template <typename T> struct Vec4;
 template <> struct Vec4<double> { using t = double4; };
 template <> struct Vec4<float> { using t = float4; };
 
+// The CTAs of a cluster that share a target chunk (jit_split) add their sums in the first
+// one: n values of this thread, at v + k * stride of its CTA's shared memory, the other
+// CTAs' values at the same place of theirs (distributed shared memory), in rank order.
+// Called by every thread of the cluster; the memory may be reused after it returns.
+__device__ __forceinline__ void cluster_sum(double* v, int stride, int n, int rank, int S)
+{
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    cl.sync();
+    if (rank == 0)
+        for (int r = 1; r < S; r++)
+        {
+            const double* o = cl.map_shared_rank(v, r);
+#pragma unroll 4
+            for (int k = 0; k < n; k++) v[k * stride] += o[k * stride];
+        }
+    cl.sync();
+}
+
 // ------------------------------------------------------------ JIT owner kernel
 
 // One CTA per chunk of <= 128 target points, 128/TPT threads, TPT targets per thread.
@@ -1001,23 +1020,23 @@ template <> struct Vec4<float> { using t = float4; };
 // src/H2Pack_matvec.c:463-539).  With T = float the products of one tile are summed
 // in FP32 and every tile sum is added to FP64 accumulators, so an FP32 sum never
 // spans more than one tile of sources.  Outputs are written once, no atomics.
-template <int KID, typename T, int NV, int KD, int TPT>
-__global__ void __launch_bounds__(128 / TPT, sizeof(T) == 4 ? 5 * TPT : 4 * TPT) k_jit(const JitTarget* __restrict__ tgts, const JitSource* __restrict__ srcs,
-                                                   const typename Vec4<T>::t* __restrict__ pts, KParam kp, int use_shift,
+template <int KID, int NV, int KD, int TPT>
+__global__ void __launch_bounds__(128 / TPT, 5 * TPT) k_jit(const JitTarget* __restrict__ tgts, const TileRec* __restrict__ tiles,
+                                                   const float4* __restrict__ pts, KParam kp, int use_shift,
                                                    const double* __restrict__ XS, double* __restrict__ PS,
-                                                   double* __restrict__ Y1)
+                                                   double* __restrict__ Y1, int S)
 {
-    using T4 = typename Vec4<T>::t;
+    using T = float;
+    using T4 = float4;
     constexpr int NT = 128 / TPT;
     constexpr int W = KD * NV;
-    constexpr bool SPLIT = sizeof(T) < sizeof(double);
-    // FP32: 64-point tiles keep shared memory at ~21 KB so 10 CTAs fit an SM
-    constexpr int TILE = (SPLIT || 128 * W * (int) sizeof(T) > 32768) ? 64 : 128;
+    constexpr int TILE = 64;   // keeps shared memory at ~21 KB, so 10 CTAs fit an SM
     __shared__ T4 s_pt[TILE];
     __shared__ T s_in[TILE * W];
     // FP64 sums of the FP32 tile sums, one column per thread (conflict-free)
-    __shared__ double s_acc[SPLIT ? TPT * W * NT : 1];
-    const JitTarget tg = tgts[blockIdx.x];
+    __shared__ double s_acc[TPT * W * NT];
+    const int rank = (int) (blockIdx.x & (S - 1));
+    const JitTarget tg = tgts[blockIdx.x / S];
     const T p0 = (T) kp.p0, c0 = (T) kp.c0;
 
     T4 xi[TPT];
@@ -1031,16 +1050,13 @@ __global__ void __launch_bounds__(128 / TPT, sizeof(T) == 4 ? 5 * TPT : 4 * TPT)
         xi[q] = pts[tg.pt0 + (valid[q] ? i : 0)];
 #pragma unroll
         for (int k = 0; k < W; k++) acc[q][k] = T(0);
-        if constexpr (SPLIT)
-        {
 #pragma unroll
-            for (int k = 0; k < W; k++) s_acc[(q * W + k) * NT + threadIdx.x] = 0.0;
-        }
+        for (int k = 0; k < W; k++) s_acc[(q * W + k) * NT + threadIdx.x] = 0.0;
     }
 
-    for (int s = tg.src_beg; s < tg.src_end; s++)
+    for (int t = tg.tile_beg + rank; t < tg.tile_end; t += S)
     {
-        const JitSource sc = srcs[s];
+        const TileRec sc = tiles[t];
         T4 xs[TPT];
 #pragma unroll
         for (int q = 0; q < TPT; q++)
@@ -1048,9 +1064,9 @@ __global__ void __launch_bounds__(128 / TPT, sizeof(T) == 4 ? 5 * TPT : 4 * TPT)
             xs[q] = xi[q];
             if (use_shift) { xs[q].x += (T) sc.sx; xs[q].y += (T) sc.sy; xs[q].z += (T) sc.sz; }
         }
-        for (int j0 = 0; j0 < sc.npt; j0 += TILE)
+        for (int j0 = 0; j0 < sc.nj; j0 += TILE)
         {
-            const int nj = min(TILE, sc.npt - j0);
+            const int nj = min(TILE, sc.nj - j0);
             __syncthreads();
             for (int j = threadIdx.x; j < nj; j += NT) s_pt[j] = pts[sc.pt0 + j0 + j];
             for (int i = threadIdx.x; i < nj * W; i += NT)
@@ -1089,19 +1105,18 @@ __global__ void __launch_bounds__(128 / TPT, sizeof(T) == 4 ? 5 * TPT : 4 * TPT)
                     }
                 }
             }
-            if constexpr (SPLIT)
-            {
 #pragma unroll
-                for (int q = 0; q < TPT; q++)
+            for (int q = 0; q < TPT; q++)
 #pragma unroll
-                    for (int k = 0; k < W; k++)
-                    {
-                        s_acc[(q * W + k) * NT + threadIdx.x] += (double) acc[q][k];
-                        acc[q][k] = T(0);
-                    }
-            }
+                for (int k = 0; k < W; k++)
+                {
+                    s_acc[(q * W + k) * NT + threadIdx.x] += (double) acc[q][k];
+                    acc[q][k] = T(0);
+                }
         }
     }
+    if (S > 1) cluster_sum(s_acc + threadIdx.x, NT, TPT * W, rank, S);
+    if (rank != 0) return;
 #pragma unroll
     for (int q = 0; q < TPT; q++)
     {
@@ -1110,10 +1125,7 @@ __global__ void __launch_bounds__(128 / TPT, sizeof(T) == 4 ? 5 * TPT : 4 * TPT)
         double* o = (tg.out_y1 ? Y1 : PS) + (long long) (tg.out_row + KD * i) * NV;
 #pragma unroll
         for (int k = 0; k < W; k++)
-        {
-            if constexpr (SPLIT) o[k] = s_acc[(q * W + k) * NT + threadIdx.x];
-            else o[k] = (double) acc[q][k];
-        }
+            o[k] = s_acc[(q * W + k) * NT + threadIdx.x];
     }
 }
 
@@ -1476,10 +1488,10 @@ __global__ void __launch_bounds__(Jit64Cfg<NV, KD>::NT, Jit64Cfg<NV, KD>::CTAS)
 // k_jit_tc; otherwise differences (exact-difference form for Coulomb, see two_sum).
 // FP32 sums per 64-source tile, FP64 across tiles.
 template <int KID, int NV, bool FAR>
-__global__ void __launch_bounds__(64, NV >= 16 ? 8 : 10) k_jit2(const JitTarget* __restrict__ tgts, const JitSource* __restrict__ srcs,
+__global__ void __launch_bounds__(64, NV >= 16 ? 8 : 10) k_jit2(const JitTarget* __restrict__ tgts, const TileRec* __restrict__ tiles,
                                                  const float4* __restrict__ pts, KParam kp,
                                                  const double* __restrict__ XS, double* __restrict__ PS,
-                                                 double* __restrict__ Y1, const float4* __restrict__ plo)
+                                                 double* __restrict__ Y1, const float4* __restrict__ plo, int S)
 {
     constexpr bool EX = KID == KRNL_COULOMB_ID && !FAR;
     constexpr int TILE = 64, NT = 64;
@@ -1487,7 +1499,8 @@ __global__ void __launch_bounds__(64, NV >= 16 ? 8 : 10) k_jit2(const JitTarget*
     __shared__ float4 s_l[EX ? TILE : 1];    // {x', x', y', y'} (EX)
     __shared__ float2 s_in[TILE * NV];       // (in, in)
     __shared__ double s_acc[2 * NV][NT];     // FP64 sums of the tile sums, [target q x NV + v][thread]
-    const JitTarget tg = tgts[blockIdx.x];
+    const int rank = (int) (blockIdx.x & (S - 1));
+    const JitTarget tg = tgts[blockIdx.x / S];
     const float p0 = (float) kp.p0, c0 = (float) kp.c0;
     float q0 = 0.f, q1 = 0.f;
     if constexpr (FAR) ScalarFar<KID>::prep(p0, c0, q0, q1);
@@ -1505,9 +1518,9 @@ __global__ void __launch_bounds__(64, NV >= 16 ? 8 : 10) k_jit2(const JitTarget*
         s_acc[NV + v][threadIdx.x] = 0.0;
     }
     const float2 m1 = make_float2(-1.f, -1.f);
-    for (int s = tg.src_beg; s < tg.src_end; s++)
+    for (int t = tg.tile_beg + rank; t < tg.tile_end; t += S)
     {
-        const JitSource sc = srcs[s];
+        const TileRec sc = tiles[t];
         const float ax = x0.x + sc.sx, ay = x0.y + sc.sy, az = x0.z + sc.sz;
         const float bx = x1.x + sc.sx, by = x1.y + sc.sy, bz = x1.z + sc.sz;
         const float2 X = make_float2(ax, bx), Y = make_float2(ay, by), Z = make_float2(az, bz);
@@ -1523,9 +1536,9 @@ __global__ void __launch_bounds__(64, NV >= 16 ? 8 : 10) k_jit2(const JitTarget*
             two_sum(x0.y, sc.sy, l0.y, YH.x, YL.x); two_sum(x1.y, sc.sy, l1.y, YH.y, YL.y);
             two_sum(x0.z, sc.sz, l0.z, ZH.x, ZL.x); two_sum(x1.z, sc.sz, l1.z, ZH.y, ZL.y);
         }
-        for (int j0 = 0; j0 < sc.npt; j0 += TILE)
+        for (int j0 = 0; j0 < sc.nj; j0 += TILE)
         {
-            const int nj = min(TILE, sc.npt - j0);
+            const int nj = min(TILE, sc.nj - j0);
             __syncthreads();
             if (threadIdx.x < nj)
             {
@@ -1585,6 +1598,8 @@ __global__ void __launch_bounds__(64, NV >= 16 ? 8 : 10) k_jit2(const JitTarget*
             }
         }
     }
+    if (S > 1) cluster_sum(&s_acc[0][threadIdx.x], NT, 2 * NV, rank, S);
+    if (rank != 0) return;
     double* o = tg.out_y1 ? Y1 : PS;
 #pragma unroll
     for (int v = 0; v < NV; v++)
@@ -1724,7 +1739,7 @@ __global__ void __launch_bounds__(256, 4) k_jit_tc(const JitTarget* __restrict__
                                                    const float4* __restrict__ pts, const float4* __restrict__ ppts,
                                                    const uint4* __restrict__ pin, KParam kp, double* __restrict__ PS,
                                                    double* __restrict__ Y1, const float4* __restrict__ plo,
-                                                   const float4* __restrict__ pplo)
+                                                   const float4* __restrict__ pplo, int S)
 {
     // EX: exact differences (Coulomb near field; plo / pplo = low parts of the points / panels)
     constexpr bool EX = KID == KRNL_COULOMB_ID && !FAR;
@@ -1732,7 +1747,8 @@ __global__ void __launch_bounds__(256, 4) k_jit_tc(const JitTarget* __restrict__
     extern __shared__ __align__(16) unsigned char jtc_raw[];
     SM& sm = *reinterpret_cast<SM*>(jtc_raw);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
-    const JitTarget tg = tgts[blockIdx.x];
+    const int rank = (int) (blockIdx.x & (S - 1));   // of the chunk's S CTAs (jit_split)
+    const JitTarget tg = tgts[blockIdx.x / S];
     const bool busy = warp * 16 < tg.npt;
     const float p0 = (float) kp.p0, c0 = (float) kp.c0;
     float q0 = 0.f, q1 = 0.f;
@@ -1770,11 +1786,11 @@ __global__ void __launch_bounds__(256, 4) k_jit_tc(const JitTarget* __restrict__
     // Pipeline over the chunk's tiles k = 0 .. nt-1: tile k is computed from buffer
     // k & 1 while tile k+1 sits in the other buffer; after the tile's barrier tile k+2
     // is copied into buffer k & 1, and the record of tile k+4 into ring slot k & 3.
-    const TileRec* rec = tiles + tg.tile_beg;
-    const int nt = tg.tile_end - tg.tile_beg;
+    const TileRec* rec = tiles + tg.tile_beg + rank;
+    const int nt = (tg.tile_end - tg.tile_beg - rank + S - 1) / S;
     auto issue_rec = [&](int k) {   // threads 0, 1: the two 16-byte halves
         if (threadIdx.x < 2 && k < nt)
-            cp_async16(reinterpret_cast<uint4*>(&sm.rec[k & 3]) + threadIdx.x, reinterpret_cast<const uint4*>(rec + k) + threadIdx.x);
+            cp_async16(reinterpret_cast<uint4*>(&sm.rec[k & 3]) + threadIdx.x, reinterpret_cast<const uint4*>(rec + (long long) k * S) + threadIdx.x);
     };
     auto issue = [&](int k, int buf) {
         if (k >= nt) return;
@@ -1894,6 +1910,9 @@ __global__ void __launch_bounds__(256, 4) k_jit_tc(const JitTarget* __restrict__
         issue_rec(k + 4);
         cp_async_commit();
     }
+    // the sums of the chunk's other CTAs, in rank order
+    if (S > 1) cluster_sum(&sm.acc[warp][0][lane], 32, 8, rank, S);
+    if (rank != 0) return;
     // accumulator (n, q) of lane (g, t): right-hand side g + 8 (q >> 1), target
     // 16w + 8n + 2t + (q & 1)
     double* base = (tg.out_y1 ? Y1 : PS) + (long long) tg.out_row * NV;
@@ -4117,7 +4136,10 @@ cudaError_t launch_asm(int NV, const AsmTask* t, int n, const int* slots, const 
 
 // CTAs per target chunk (the CTAs of a cluster share a chunk's source tiles): the smallest
 // power of two that gives the launch two waves of the SMs' CTA slots, at most 8 (the portable
-// cluster size).
+// cluster size).  Two waves: with one, near fields of 1,063 chunks (FP64, N = 120,000) took
+// 2.23 instead of 2.05 ms and the served case below 38.1 instead of 37.4; with four, a far
+// field of 1,216 chunks 10.9 instead of 9.6 ms.  FP32: 16 requests on a Gaussian matrix of N =
+// 20,011 (192 near chunks on 592 slots): 60.8 -> 37.4 ms.
 static int jit_split(int n, int per_sm)
 {
     int S = 1;
@@ -4145,13 +4167,14 @@ static cudaError_t launch_cluster(void (*kern)(P...), int n, int S, int threads,
 }
 
 template <int KID, typename T, int KD>
-static cudaError_t launch_jit_k(int NV, const JitTarget* tg, int n, const JitSource* sr, const void* pts, KParam kp,
+static cudaError_t launch_jit_k(int NV, const JitTarget* tg, int n, const void* pts, KParam kp,
                                 int use_shift, int use_tc, const double* XS, double* PS, double* Y1, cudaStream_t st,
                                 int far, const float4* ppts, const uint4* pin, const TileRec* tiles,
                                 const float4* lo, const float4* plo)
 {
     using T4 = typename Vec4<T>::t;
     const T4* p = (const T4*) pts;
+    if (!tiles) return cudaErrorInvalidValue;
     // the FP32 Coulomb near field reads the low parts of the points
     if (KID == KRNL_COULOMB_ID && sizeof(T) == 4 && !far && !lo) return cudaErrorInvalidValue;
     // FP32 scalar kernels on panels of 8 or 16: right-hand-side products on the tensor
@@ -4160,8 +4183,8 @@ static cudaError_t launch_jit_k(int NV, const JitTarget* tg, int n, const JitSou
     {
         if (use_tc && (NV == 16 || NV == 8) && use_shift)
         {
-            // the tensor-core kernel reads the source panels and tile lists
-            if (!ppts || !pin || !tiles) return cudaErrorInvalidValue;
+            // the tensor-core kernel reads the source panels
+            if (!ppts || !pin) return cudaErrorInvalidValue;
             if (KID == KRNL_COULOMB_ID && !far && !plo) return cudaErrorInvalidValue;
             const float4* p4 = (const float4*) pts;
             const int b = jit_tc_smem_bytes(KID == KRNL_COULOMB_ID && !far);
@@ -4171,8 +4194,8 @@ static cudaError_t launch_jit_k(int NV, const JitTarget* tg, int n, const JitSou
                                  : (far ? k_jit_tc<KID, 8, true> : k_jit_tc<KID, 8, false>);
             cudaError_t e = allow_smem(kern, b);
             if (e != cudaSuccess) return e;
-            kern<<<n, 256, b, st>>>(tg, tiles, p4, ppts, pin, kp, PS, Y1, lo, plo);
-            return cudaGetLastError();
+            const int S = jit_split(n, 4);
+            return launch_cluster(kern, n, S, 256, b, st, tg, tiles, p4, ppts, pin, kp, PS, Y1, lo, plo, S);
         }
     }
     // FP32: two targets per thread (64 threads per 128-point chunk) where the accumulators
@@ -4183,7 +4206,6 @@ static cudaError_t launch_jit_k(int NV, const JitTarget* tg, int n, const JitSou
             return cudaErrorInvalidValue;   // tensor kernels run in panels of <= 8 right-hand sides
         else if constexpr (sizeof(T) == 8)
         {
-            if (!tiles) return cudaErrorInvalidValue;
             const int S = jit_split(n, 4);
             return launch_cluster(k_jit64<KID, NVc, KD>, n, S, Jit64Cfg<NVc, KD>::NT, 0, st, tg, tiles, p, kp, XS, PS, Y1, S);
         }
@@ -4191,24 +4213,27 @@ static cudaError_t launch_jit_k(int NV, const JitTarget* tg, int n, const JitSou
         {
             // scalar FP32 kernels: the two targets of a thread as one FP32x2 pair
             if (!use_shift) return cudaErrorInvalidValue;   // FP32 evaluation is re-centred
-            if (far) k_jit2<KID, NVc, true><<<n, 64, 0, st>>>(tg, sr, (const float4*) pts, kp, XS, PS, Y1, lo);
-            else k_jit2<KID, NVc, false><<<n, 64, 0, st>>>(tg, sr, (const float4*) pts, kp, XS, PS, Y1, lo);
+            const int S = jit_split(n, 8);
+            return launch_cluster(far ? k_jit2<KID, NVc, true> : k_jit2<KID, NVc, false>, n, S, 64, 0, st, tg, tiles,
+                                  (const float4*) pts, kp, XS, PS, Y1, lo, S);
         }
-        else if constexpr (KD * NVc <= 16 && sizeof(T) == 4)
-            k_jit<KID, T, NVc, KD, 2><<<n, 64, 0, st>>>(tg, sr, p, kp, use_shift, XS, PS, Y1);
         else
-            k_jit<KID, T, NVc, KD, 1><<<n, 128, 0, st>>>(tg, sr, p, kp, use_shift, XS, PS, Y1);
+        {
+            constexpr int TPT = KD * NVc <= 16 ? 2 : 1;
+            const int S = jit_split(n, 5 * TPT);
+            return launch_cluster(k_jit<KID, NVc, KD, TPT>, n, S, 128 / TPT, 0, st, tg, tiles, p, kp, use_shift, XS, PS, Y1, S);
+        }
     });
-    return cudaGetLastError();
+    return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_jit(int kid, int fp32, int NV, const JitTarget* tg, int n, const JitSource* sr, const void* pts,
+cudaError_t launch_jit(int kid, int fp32, int NV, const JitTarget* tg, int n, const void* pts,
                        KParam kp, int use_shift, int use_tc, const double* XS, double* PS, double* Y1, cudaStream_t st,
                        int far, const float4* ppts, const uint4* pin, const TileRec* tiles, const float4* lo,
                        const float4* plo)
 {
     if (n <= 0) return cudaSuccess;
-#define H2G_JIT_ARGS NV, tg, n, sr, pts, kp, use_shift, use_tc, XS, PS, Y1, st, far, ppts, pin, tiles, lo, plo
+#define H2G_JIT_ARGS NV, tg, n, pts, kp, use_shift, use_tc, XS, PS, Y1, st, far, ppts, pin, tiles, lo, plo
     switch (kid)
     {
         case KRNL_COULOMB_ID:  return fp32 ? launch_jit_k<KRNL_COULOMB_ID, float, 1>(H2G_JIT_ARGS)

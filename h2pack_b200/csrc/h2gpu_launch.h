@@ -34,11 +34,11 @@ cudaError_t launch_y1sum(int NV, const Y1Task* t, int n, const int* slots, const
                          cudaStream_t st);
 cudaError_t launch_asm(int NV, const AsmTask* t, int n, const int* slots, const double* PS, const int* fwd,
                        double* Y, long long y_rs, long long y_cs, int nv, long long rows, cudaStream_t st);
-// far: every source set is admissible for its target (r > 0); ppts / pin / tiles: the
-// source panels and tile lists, which the tensor-core kernel (FP32 scalar kernels,
-// NV 8 / 16, use_tc) reads; lo / plo: the low parts of the FP32 points and of the
+// far: every source set is admissible for its target (r > 0); tiles: the source tiles of
+// the targets; ppts / pin: the source panels, which the tensor-core kernel (FP32 scalar
+// kernels, NV 8 / 16, use_tc) reads; lo / plo: the low parts of the FP32 points and of the
 // panels, which the FP32 Coulomb near field needs (exact differences)
-cudaError_t launch_jit(int kid, int fp32, int NV, const JitTarget* tg, int n, const JitSource* sr, const void* pts,
+cudaError_t launch_jit(int kid, int fp32, int NV, const JitTarget* tg, int n, const void* pts,
                        KParam kp, int use_shift, int use_tc, const double* XS, double* PS, double* Y1, cudaStream_t st,
                        int far = 0, const float4* ppts = nullptr, const uint4* pin = nullptr,
                        const TileRec* tiles = nullptr, const float4* lo = nullptr, const float4* plo = nullptr);

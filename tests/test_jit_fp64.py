@@ -30,3 +30,24 @@ def test_matches_64_bit_product(kernel, param, n, leaf):
         torch.cuda.synchronize()
         assert float((y - Y[:, :nv]).norm() / Y[:, :nv].norm()) < 1e-13, nv
     img.close()
+
+
+@pytest.mark.parametrize("kernel", ["coulomb", "gaussian", "matern32", "rpy"])
+@pytest.mark.parametrize("n,leaf", [(40, 100), (1500, 300), (9000, 100)])
+def test_mixed_small_images(kernel, n, leaf):
+    """FP32 evaluation with clusters of 2 to 8 CTAs per chunk, every panel width, on the CUDA
+    and the tensor cores: the mixed path's 2e-6 (FP32 kernel values, 3xTF32 products)."""
+    import torch
+    from perf import cases
+    case = {"kind": "apply", "kernel": kernel, "n": n, "leaf": leaf, "mode": "jit", "precision": "mixed", "api": "device"}
+    rep = cases.Rep(case, n, 3)
+    img = cases.Image(rep.describe(), "mixed")
+    X = cases._rhs(case, rep.kd * n, 16, 3)
+    Y = rep.apply(X)
+    for variant in ("tc", "simt"):
+        img.set_jit_variant(variant)
+        for nv in (1, 2, 4, 5, 8, 16):
+            y = img.matmul_device(X[:, :nv].contiguous())
+            torch.cuda.synchronize()
+            assert float((y - Y[:, :nv]).norm() / Y[:, :nv].norm()) < 2e-6, (variant, nv)
+    img.close()
