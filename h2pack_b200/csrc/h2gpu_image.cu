@@ -90,6 +90,8 @@ struct h2gpu_image {
     std::mutex mu;
     int device = 0;
     cudaStream_t stream = nullptr;
+    cudaStream_t chain = nullptr;            // the sweeps and the far field, beside the near field (run_panel)
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     int precision = H2GPU_PREC_FP64;
     int max_nv = 16;
 
@@ -210,6 +212,9 @@ void free_all(h2gpu_image* im)
         if (e) cudaEventDestroy(e);
     if (im->graph_exec) cudaGraphExecDestroy(im->graph_exec);
     if (im->graph) cudaGraphDestroy(im->graph);
+    if (im->ev_fork) cudaEventDestroy(im->ev_fork);
+    if (im->ev_join) cudaEventDestroy(im->ev_join);
+    if (im->chain) cudaStreamDestroy(im->chain);
     if (im->stream) cudaStreamDestroy(im->stream);
 }
 
@@ -1803,13 +1808,19 @@ bool panels_used(const h2gpu_image* im, int NV)
     return im->BD_JIT && im->kd == 1 && im->jit_tc && im->d_pin && (NV == 8 || NV == 16);
 }
 
+// Whether a panel takes the pair plan (each unordered JIT pair evaluated once).
+bool pair_plan(const h2gpu_image* im, int NV)
+{
+    return im->has_pair && im->jit_pair && im->precision == H2GPU_PREC_MIXED && im->jit_tc && (NV == 8 || NV == 16);
+}
+
 // One panel of NV right-hand sides: X (original order, strides x_rs, x_cs) -> Y.
 int run_panel(h2gpu_image* im, int NV, int nv, const double* X, long long x_rs, long long x_cs, double* Y,
               long long y_rs, long long y_cs, cudaStream_t s, bool timed)
 {
     const bool f32 = im->precision == H2GPU_PREC_MIXED;
     cudaEvent_t* e = im->ev.e;
-    if (im->has_pair && im->jit_pair && f32 && im->jit_tc && (NV == 8 || NV == 16))
+    if (pair_plan(im, NV))
     {
         // each unordered JIT pair evaluated once, applied both ways (tensor cores)
         const KParam kp = kparam_of(im);
@@ -1849,12 +1860,73 @@ int run_panel(h2gpu_image* im, int NV, int nv, const double* X, long long x_rs, 
         return H2GPU_OK;
     }
     const bool wide = f32 && !im->BD_JIT && NV == 64;   // two GEMM passes per block list
+    const bool panels = f32 && panels_used(im, NV);
     const long long xs_rows = (long long) im->N + im->y0_rows;
+    // The near field (D) reads the input only, and only the assembly reads its results: it
+    // runs on the caller's stream while the chain of dependent launches -- upward sweep,
+    // far field, downward sweep, one or two launches per tree level, which leave much of
+    // the GPU idle -- runs on the image's chain stream, whose higher priority lets its CTAs
+    // in as near-field CTAs retire.  Coulomb N = 80,000, stored, one right-hand side: FP64 1.09
+    // -> 1.01 ms, mixed 0.67 -> 0.58; Gaussian N = 10,007 on the fly, FP64: 0.30 -> 0.23; 12
+    // batched Gaussian matrices, 8 right-hand sides, mixed: 1.16 -> 0.95; Matern N = 125,000, 16,
+    // mixed: 3.98 -> 3.68.  The FP64 on-the-fly near field, bound by the FP64 pipe that the
+    // sweep needs too, starts after the upward sweep (Coulomb N = 30,011, 3 right-hand sides:
+    // 0.92 one after the other, 0.99 from the fork on, 0.84 so); stored blocks and FP32 gain
+    // from the fork on (Coulomb N = 80,000, FP64: 1.01 against 1.05 ms).
+    cudaStream_t c = im->chain;
     if (timed) CK(cudaEventRecord(e[0], s));
     CK(launch_gather(NV, X, x_rs, x_cs, nv, im->d_fwd, im->N, im->d_XS, s));
     if (wide) CK(launch_split3(im->d_XS, 0, im->N, xs_rows, im->d_XS3, s));
-    // D phase first: it needs only x (in the graph-free stream order it simply runs before the upward sweep)
+    if (panels) CK(launch_panel_in(NV, im->d_pg, 0, im->n_pg_pts, im->d_XS, im->d_pin, s));
+    CK(cudaEventRecord(im->ev_fork, s));
     if (timed) CK(cudaEventRecord(e[1], s));
+    CK(cudaStreamWaitEvent(c, im->ev_fork, 0));
+    for (size_t L = 0; L + 1 < im->up_beg.size(); L++)
+    {
+        int b = im->up_beg[L], n = im->up_beg[L + 1] - b;
+        if (f32) CK(launch_up<float>(NV, im->d_up + b, n, im->d_U32, im->d_XS, c, sweep_tc(im)));
+        else CK(launch_up<double>(NV, im->d_up + b, n, im->d_U64, im->d_XS, c));
+    }
+    if (timed) CK(cudaEventRecord(e[3], c));
+    if (im->BD_JIT && !f32)
+    {
+        CK(cudaEventRecord(im->ev_join, c));
+        CK(cudaStreamWaitEvent(s, im->ev_join, 0));
+        if (timed) CK(cudaEventRecord(e[1], s));
+    }
+    if (!im->BD_JIT)
+    {
+        if (wide)
+        {
+            const int* nw = im->n_wide;
+            CK(launch_split3(im->d_XS, im->N, im->y0_rows, xs_rows, im->d_XS3, c));   // the skeleton rows y0
+            CK(launch_blk_wide(0, im->d_blkB, im->d_wide, nw[0], im->d_B32, im->d_XS3, xs_rows, im->d_PS, c,
+                               im->d_status));
+            CK(launch_blk_wide(1, im->d_blkB, im->d_wide + nw[0], nw[1], im->d_B32, im->d_XS3, xs_rows, im->d_PS, c,
+                               im->d_status));
+            im->st.n_launches += 2;   // the second pass and the split of the inputs
+        }
+        else if (f32) CK(launch_blk<float>(NV, im->d_blkB, im->n_blkB, im->d_B32, im->d_XS, im->d_PS, c, im->blk_tc, im->d_status,
+                                           im->blk1_small[0][1]));
+        else CK(launch_blk<double>(NV, im->d_blkB, im->n_blkB, im->d_B64, im->d_XS, im->d_PS, c, 0, nullptr,
+                                   im->blk1_small[0][0]));
+        CK(launch_y1sum(NV, im->d_y1t, im->n_y1, im->d_y1_slots, im->d_PS, im->d_Y1, im->y0_rows, c));
+    } else {
+        if (panels) CK(launch_panel_in(NV, im->d_pg, im->n_pg_pts, im->n_pg - im->n_pg_pts, im->d_XS, im->d_pin, c));
+        CK(launch_jit(im->kernel_id, f32, NV, im->d_jtF, im->n_jtF, f32 ? (const void*) im->d_pts32 : (const void*) im->d_pts64,
+                      kparam_of(im), f32 ? 1 : 0, im->jit_tc, im->d_XS, im->d_PS, im->d_Y1, c, im->far_diff ? 0 : 1,
+                      im->d_ppts, im->d_pin, im->d_tiles, im->d_pts32lo, im->d_pplo));
+    }
+    if (timed) CK(cudaEventRecord(e[4], c));
+    for (size_t L = 0; L + 1 < im->dn_beg.size(); L++)
+    {
+        int b = im->dn_beg[L], n = im->dn_beg[L + 1] - b;
+        if (f32) CK(launch_down<float>(NV, im->d_dn + b, n, im->d_U32, im->d_Y1, im->d_PS, im->d_PUSH, c, sweep_tc(im)));
+        else CK(launch_down<double>(NV, im->d_dn + b, n, im->d_U64, im->d_Y1, im->d_PS, im->d_PUSH, c));
+    }
+    if (timed) CK(cudaEventRecord(e[5], c));
+    CK(cudaEventRecord(im->ev_join, c));
+    // the near field, on the caller's stream
     if (!im->BD_JIT)
     {
         if (wide)
@@ -1871,56 +1943,15 @@ int run_panel(h2gpu_image* im, int NV, int nv, const double* X, long long x_rs, 
         else CK(launch_blk<double>(NV, im->d_blkD, im->n_blkD, im->d_D64, im->d_XS, im->d_PS, s, 0, nullptr,
                                    im->blk1_small[1][0]));
     } else {
-        const bool panels = f32 && panels_used(im, NV);
-        if (panels) CK(launch_panel_in(NV, im->d_pg, 0, im->n_pg_pts, im->d_XS, im->d_pin, s));
         CK(launch_jit(im->kernel_id, f32, NV, im->d_jtN, im->n_jtN, f32 ? (const void*) im->d_pts32 : (const void*) im->d_pts64,
                       kparam_of(im), f32 ? 1 : 0, im->jit_tc, im->d_XS, im->d_PS, im->d_Y1, s, 0, im->d_ppts, im->d_pin, im->d_tiles,
                       im->d_pts32lo, im->d_pplo));
-        im->st.n_launches += panels ? 1 : 0;
+        im->st.n_launches += panels ? 2 : 0;
     }
     if (timed) CK(cudaEventRecord(e[2], s));
-    for (size_t L = 0; L + 1 < im->up_beg.size(); L++)
-    {
-        int b = im->up_beg[L], n = im->up_beg[L + 1] - b;
-        if (f32) CK(launch_up<float>(NV, im->d_up + b, n, im->d_U32, im->d_XS, s, sweep_tc(im)));
-        else CK(launch_up<double>(NV, im->d_up + b, n, im->d_U64, im->d_XS, s));
-    }
-    if (timed) CK(cudaEventRecord(e[3], s));
-    if (!im->BD_JIT)
-    {
-        if (wide)
-        {
-            const int* nw = im->n_wide;
-            CK(launch_split3(im->d_XS, im->N, im->y0_rows, xs_rows, im->d_XS3, s));   // the skeleton rows y0
-            CK(launch_blk_wide(0, im->d_blkB, im->d_wide, nw[0], im->d_B32, im->d_XS3, xs_rows, im->d_PS, s,
-                               im->d_status));
-            CK(launch_blk_wide(1, im->d_blkB, im->d_wide + nw[0], nw[1], im->d_B32, im->d_XS3, xs_rows, im->d_PS, s,
-                               im->d_status));
-            im->st.n_launches += 2;   // the second pass and the split of the inputs
-        }
-        else if (f32) CK(launch_blk<float>(NV, im->d_blkB, im->n_blkB, im->d_B32, im->d_XS, im->d_PS, s, im->blk_tc, im->d_status,
-                                           im->blk1_small[0][1]));
-        else CK(launch_blk<double>(NV, im->d_blkB, im->n_blkB, im->d_B64, im->d_XS, im->d_PS, s, 0, nullptr,
-                                   im->blk1_small[0][0]));
-        CK(launch_y1sum(NV, im->d_y1t, im->n_y1, im->d_y1_slots, im->d_PS, im->d_Y1, im->y0_rows, s));
-    } else {
-        const bool panels = f32 && panels_used(im, NV);
-        if (panels) CK(launch_panel_in(NV, im->d_pg, im->n_pg_pts, im->n_pg - im->n_pg_pts, im->d_XS, im->d_pin, s));
-        CK(launch_jit(im->kernel_id, f32, NV, im->d_jtF, im->n_jtF, f32 ? (const void*) im->d_pts32 : (const void*) im->d_pts64,
-                      kparam_of(im), f32 ? 1 : 0, im->jit_tc, im->d_XS, im->d_PS, im->d_Y1, s, im->far_diff ? 0 : 1,
-                      im->d_ppts, im->d_pin, im->d_tiles, im->d_pts32lo, im->d_pplo));
-        im->st.n_launches += panels ? 1 : 0;
-    }
-    if (timed) CK(cudaEventRecord(e[4], s));
-    for (size_t L = 0; L + 1 < im->dn_beg.size(); L++)
-    {
-        int b = im->dn_beg[L], n = im->dn_beg[L + 1] - b;
-        if (f32) CK(launch_down<float>(NV, im->d_dn + b, n, im->d_U32, im->d_Y1, im->d_PS, im->d_PUSH, s, sweep_tc(im)));
-        else CK(launch_down<double>(NV, im->d_dn + b, n, im->d_U64, im->d_Y1, im->d_PS, im->d_PUSH, s));
-    }
-    if (timed) CK(cudaEventRecord(e[5], s));
+    CK(cudaStreamWaitEvent(s, im->ev_join, 0));
     CK(launch_asm(NV, im->d_asm, im->n_asm, im->d_asm_slots, im->d_PS, im->d_fwd, Y, y_rs, y_cs, nv, im->N,
-                      s));
+                  s));
     if (timed && uses_status(im, NV))
         CK(cudaMemcpyAsync(im->h_status, im->d_status, sizeof(int), cudaMemcpyDeviceToHost, s));
     if (timed) CK(cudaEventRecord(e[6], s));
@@ -2030,22 +2061,32 @@ int apply_device(h2gpu_image* im, int n_vec, const double* X, long long x_rs, lo
         pst = prepare(im, NV);
     }
     TRY(pst);
-    float ph[5] = {0, 0, 0, 0, 0};
+    float ph[5] = {0, 0, 0, 0, 0}, total = 0.f;
     for (int c0 = 0; c0 < n_vec; c0 += NV)
     {
         int nv = std::min(NV, n_vec - c0);
         TRY(run_panel(im, NV, nv, X + c0 * x_cs, x_rs, x_cs, Y + c0 * y_cs, y_rs, y_cs, s, true));
         CK(cudaEventSynchronize(im->ev.e[6]));
         TRY(check_status(im));
-        float t[6];
-        for (int k = 0; k < 6; k++) CK(cudaEventElapsedTime(&t[k], im->ev.e[k], im->ev.e[k + 1]));
-        ph[0] += t[0] + t[2];   // gather + upward
-        ph[1] += t[3];          // B
-        ph[2] += t[4];          // downward
-        ph[3] += t[1];          // D
-        ph[4] += t[5];          // assemble
+        // the pair plan runs D (1 -> 2) before the chain (2 -> 3 -> 4 -> 5), otherwise both
+        // start after the gather (1) and the assembly follows the later one
+        cudaEvent_t* ev = im->ev.e;
+        const bool pair = pair_plan(im, NV);
+        auto ms = [&](int a, int b) {
+            float t = 0.f;
+            cudaEventElapsedTime(&t, ev[a], ev[b]);
+            return t;
+        };
+        const bool after_up = im->BD_JIT && im->precision == H2GPU_PREC_FP64;   // D's start: run_panel
+        ph[0] += pair ? ms(0, 1) + ms(2, 3) : after_up ? ms(0, 3) : ms(0, 1) + ms(1, 3);   // gather + upward
+        ph[1] += ms(3, 4);                         // B
+        ph[2] += ms(4, 5);                         // downward
+        ph[3] += ms(1, 2);                         // D
+        ph[4] += std::min(ms(5, 6), ms(2, 6));     // assemble
+        total += ms(0, 6);
     }
-    for (int k = 0; k < 5; k++) { im->st.ms_phase[k] += ph[k]; im->st.ms_total += ph[k]; }
+    for (int k = 0; k < 5; k++) im->st.ms_phase[k] += ph[k];
+    im->st.ms_total += total;
     im->st.n_matvec += n_vec;
     return H2GPU_OK;
 }
@@ -2152,7 +2193,16 @@ H2G_API int h2gpu_image_create(const h2gpu_desc* desc, const h2gpu_options* opt,
     int st = H2GPU_OK;
     do {
         if (cudaSetDevice(im->device) != cudaSuccess) { st = fail(H2GPU_ERR_CUDA, "cudaSetDevice(%d) failed", im->device); break; }
-        if (cudaStreamCreateWithFlags(&im->stream, cudaStreamNonBlocking) != cudaSuccess) { st = fail(H2GPU_ERR_CUDA, "stream creation failed"); break; }
+        int prio_least = 0, prio_most = 0;
+        if (cudaStreamCreateWithFlags(&im->stream, cudaStreamNonBlocking) != cudaSuccess ||
+            cudaDeviceGetStreamPriorityRange(&prio_least, &prio_most) != cudaSuccess ||
+            cudaStreamCreateWithPriority(&im->chain, cudaStreamNonBlocking, prio_most) != cudaSuccess ||
+            cudaEventCreateWithFlags(&im->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
+            cudaEventCreateWithFlags(&im->ev_join, cudaEventDisableTiming) != cudaSuccess)
+        {
+            st = fail(H2GPU_ERR_CUDA, "stream creation failed");
+            break;
+        }
         for (auto& ev : im->ev.e)
             if (cudaEventCreate(&ev) != cudaSuccess) { st = fail(H2GPU_ERR_CUDA, "event creation failed"); break; }
         if (st != H2GPU_OK) break;
