@@ -5,7 +5,7 @@
 // (examples/PCG/pcg.c:11-152) on the shifted operator of
 // examples/SPDHSS-H2/pcg_tests.c:13-20, run for up to 16 right-hand sides ("slots")
 // at once: the slots are the columns of one 16-wide panel, so every iteration is one
-// H2 matmul (of the panel's columns up to the highest busy slot) plus five small
+// H2 matmul (of the panel's columns up to the highest busy slot) plus three small
 // kernels (direction update, p'Ap, alpha, x/r update with ||r||^2, status).  The host only enqueues iterations and reads the
 // 16 slot records once per batch of iterations; it never waits per iteration.
 //
@@ -60,15 +60,20 @@ struct CgCtx {
     double* part;       // [G][kS]
     CgSlot* sl;
     double* hist;       // [kS][kHist]
+    int* count;         // blocks done of the reduction in flight (zero between launches)
 };
 
 __device__ __forceinline__ bool running_pcg(const CgSlot& s) { return s.state == H2GPU_CG_RUN && s.kind == H2GPU_CG_PCG; }
 
 // Fixed-order reduction of per-thread column sums (thread t: column t % 16, row lane
-// t / 16) into part[blockIdx.x][col].  256 threads.
-__device__ __forceinline__ void block_col_reduce(double v, double* part)
+// t / 16) into part[blockIdx.x][col].  256 threads.  True in every thread of the block that
+// finishes last: it sees all blocks' parts (sum_parts) and takes the scalar step that follows
+// the reduction, which was a launch of its own (8.7 us of one block each, twice an
+// iteration) before.
+__device__ __forceinline__ bool block_col_reduce(double v, const CgCtx& c)
 {
     __shared__ double s[256];
+    __shared__ int last;
     s[threadIdx.x] = v;
     __syncthreads();
     for (int w = 128; w >= kS; w >>= 1)
@@ -76,7 +81,20 @@ __device__ __forceinline__ void block_col_reduce(double v, double* part)
         if (threadIdx.x < w) s[threadIdx.x] += s[threadIdx.x + w];
         __syncthreads();
     }
-    if (threadIdx.x < kS) part[blockIdx.x * kS + threadIdx.x] = s[threadIdx.x];
+    if (threadIdx.x < kS)
+    {
+        c.part[blockIdx.x * kS + threadIdx.x] = s[threadIdx.x];
+        __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        last = atomicAdd(c.count, 1) == (int) gridDim.x - 1;
+        if (last) *c.count = 0;
+        __threadfence();
+    }
+    __syncthreads();
+    return last != 0;
 }
 
 // Row range of block b: contiguous, fixed by N and G only.
@@ -94,7 +112,8 @@ __device__ __forceinline__ double sum_parts(const double* part, int G)
     __shared__ double s[256];
     const int col = threadIdx.x / kS, j = threadIdx.x % kS;   // 16 threads per column
     double v = 0.0;
-    for (int b = j; b < G; b += kS) v += part[b * kS + col];
+#pragma unroll 8
+    for (int b = j; b < G; b += kS) v += __ldcg(part + b * kS + col);
     s[threadIdx.x] = v;
     __syncthreads();
     double tot = 0.0;
@@ -139,12 +158,8 @@ __global__ void k_cg_dot(CgCtx c)
             const double p = c.P[e];
             v += p * (c.AP[e] + c.mu * p);
         }
-    block_col_reduce(v, c.part);
-}
-
-__global__ void k_cg_alpha(CgCtx c)
-{
-    const double pap = sum_parts(c.part, c.G);
+    if (!block_col_reduce(v, c)) return;
+    const double pap = sum_parts(c.part, c.G);   // alpha = rho / p.Ap
     if (threadIdx.x < kS)
     {
         CgSlot& s = c.sl[threadIdx.x];
@@ -177,11 +192,8 @@ __global__ void k_cg_update(CgCtx c)
             c.X[e] = c.AP[e] + c.mu * c.P[e];
         }
     }
-    block_col_reduce(v, c.part);
-}
-
-__global__ void k_cg_finish(CgCtx c)
-{
+    // the slots' records after the iteration
+    if (!block_col_reduce(v, c)) return;
     const double rr = sum_parts(c.part, c.G);
     if (threadIdx.x < kS)
     {
@@ -221,11 +233,7 @@ __global__ void k_cg_resid(CgCtx c)
             c.R[e] = r;
             v += r * r;
         }
-    block_col_reduce(v, c.part);
-}
-
-__global__ void k_cg_check_finish(CgCtx c)
-{
+    if (!block_col_reduce(v, c)) return;
     const double rr = sum_parts(c.part, c.G);
     if (threadIdx.x < kS)
     {
@@ -246,41 +254,57 @@ __global__ void k_cg_check_finish(CgCtx c)
     }
 }
 
-// ||b||^2 of a new slot and its record (one block of 256 threads).
-__global__ void k_cg_admit(CgCtx c, int slot, int kind, double tol, int max_iter, int restart)
+// A new slot: its columns of the panels, ||b||^2 and its record.  One launch over the rows;
+// the columns were five strided copies of 8-byte elements before, and ||b||^2 one block's.
+__global__ void k_cg_admit(CgCtx c, const double* __restrict__ d_b, int slot, int kind, double tol, int max_iter, int restart)
 {
-    __shared__ double s[256];
+    int r0, r1;
+    rows_of(c.N, c.G, blockIdx.x, r0, r1);
+    double* B = const_cast<double*>(c.B);
     double v = 0.0;
-    for (int i = threadIdx.x; i < c.N; i += 256)
+    for (int i = r0 + threadIdx.x; i < r1; i += 256)
     {
-        const double b = c.B[(long long) i * kS + slot];
+        const long long e = (long long) i * kS + slot;
+        const double b = d_b[i];
+        B[e] = b;
+        c.R[e] = b;
+        c.X[e] = 0.0;
+        c.P[e] = kind == H2GPU_CG_MATVEC ? b : 0.0;
         v += b * b;
     }
-    s[threadIdx.x] = v;
+    // block_col_reduce gives sixteen partial sums of the block: of threads t, t + 16, ..
+    if (!block_col_reduce(v, c)) return;
+    const double col = sum_parts(c.part, c.G);
+    __shared__ double s[kS];
+    if (threadIdx.x < kS) s[threadIdx.x] = col;
     __syncthreads();
-    for (int w = 128; w > 0; w >>= 1)
-    {
-        if (threadIdx.x < w) s[threadIdx.x] += s[threadIdx.x + w];
-        __syncthreads();
-    }
     if (threadIdx.x == 0)
     {
+        double b2 = 0.0;
+        for (int k = 0; k < kS; k++) b2 += s[k];
         CgSlot r;
         memset(&r, 0, sizeof(r));
-        r.bnorm2 = s[0];
-        r.tol2 = tol * tol * s[0];
-        r.rho = r.rho_prev = r.rr = s[0];
+        r.bnorm2 = b2;
+        r.tol2 = tol * tol * b2;
+        r.rho = r.rho_prev = r.rr = b2;
         r.kind = kind;
         r.max_iter = max_iter;
         r.restart = restart;
         r.first = 1;
         // b = 0: x = 0 is the solution (pcg.c's loop does not start)
-        r.state = (kind == H2GPU_CG_PCG && s[0] == 0.0) ? H2GPU_CG_DONE : H2GPU_CG_RUN;
+        r.state = (kind == H2GPU_CG_PCG && b2 == 0.0) ? H2GPU_CG_DONE : H2GPU_CG_RUN;
         c.sl[slot] = r;
     }
 }
 
 __global__ void k_cg_free(CgSlot* sl, int slot) { sl[slot].state = H2GPU_CG_FREE; }
+
+// A finished slot's solution, and the slot free again
+__global__ void k_cg_take(CgCtx c, int slot, double* __restrict__ d_x)
+{
+    for (int i = blockIdx.x * 256 + threadIdx.x; i < c.N; i += gridDim.x * 256) d_x[i] = c.X[(long long) i * kS + slot];
+    if (blockIdx.x == 0 && threadIdx.x == 0) c.sl[slot].state = H2GPU_CG_FREE;
+}
 
 }  // namespace
 
@@ -333,7 +357,7 @@ H2G_API int h2gpu_cg_create(h2gpu_image* img, double mu, int refresh, h2gpu_cg**
     do {
         if (cudaSetDevice(g->device) != cudaSuccess) { stc = h2gpu::set_error(H2GPU_ERR_CUDA, "cudaSetDevice failed"); break; }
         const size_t panel = (size_t) N * kS;
-        if (cudaMalloc(&g->mem, sizeof(double) * (5 * panel + (size_t) G * kS)) != cudaSuccess ||
+        if (cudaMalloc(&g->mem, sizeof(double) * (5 * panel + (size_t) G * kS) + sizeof(int)) != cudaSuccess ||
             cudaMalloc(&g->d_sl, sizeof(CgSlot) * kS) != cudaSuccess ||
             cudaMalloc(&g->d_hist, sizeof(double) * kS * kHist) != cudaSuccess ||
             cudaMallocHost(&g->h_sl, sizeof(CgSlot) * kS) != cudaSuccess ||
@@ -346,9 +370,11 @@ H2G_API int h2gpu_cg_create(h2gpu_image* img, double mu, int refresh, h2gpu_cg**
         double* m = g->mem;
         g->c.B = m; g->c.X = m + panel; g->c.R = m + 2 * panel; g->c.P = m + 3 * panel; g->c.AP = m + 4 * panel;
         g->c.part = m + 5 * panel;
+        g->c.count = (int*) (g->c.part + (size_t) G * kS);
         g->c.sl = g->d_sl;
         g->c.hist = g->d_hist;
         if (cudaMemsetAsync(g->mem, 0, sizeof(double) * 5 * panel, g->stream) != cudaSuccess ||
+            cudaMemsetAsync(g->c.count, 0, sizeof(int), g->stream) != cudaSuccess ||
             cudaMemsetAsync(g->d_sl, 0, sizeof(CgSlot) * kS, g->stream) != cudaSuccess ||
             cudaStreamSynchronize(g->stream) != cudaSuccess)
         {
@@ -386,17 +412,8 @@ H2G_API int h2gpu_cg_admit(h2gpu_cg* g, int slot, int kind, const double* d_b, d
     std::lock_guard<std::mutex> lk(g->lock);
     if (g->h_sl[slot].state != H2GPU_CG_FREE) return h2gpu::set_error(H2GPU_ERR_STATE, "slot is busy");
     CGCK(cudaSetDevice(g->device));
-    const size_t pitch = sizeof(double) * kS, col = sizeof(double);
-    double* B = const_cast<double*>(g->c.B);
-    CGCK(cudaMemcpy2DAsync(B + slot, pitch, d_b, col, col, g->N, cudaMemcpyDeviceToDevice, g->stream));
-    CGCK(cudaMemcpy2DAsync(g->c.R + slot, pitch, d_b, col, col, g->N, cudaMemcpyDeviceToDevice, g->stream));
-    CGCK(cudaMemset2DAsync(g->c.X + slot, pitch, 0, col, g->N, g->stream));
-    if (kind == H2GPU_CG_MATVEC)
-        CGCK(cudaMemcpy2DAsync(g->c.P + slot, pitch, d_b, col, col, g->N, cudaMemcpyDeviceToDevice, g->stream));
-    else
-        CGCK(cudaMemset2DAsync(g->c.P + slot, pitch, 0, col, g->N, g->stream));
     const int restart = g->precision == H2GPU_PREC_FP64 ? 0 : g->refresh;
-    k_cg_admit<<<1, 256, 0, g->stream>>>(g->c, slot, kind, tol, max_iter, restart);
+    k_cg_admit<<<g->c.G, 256, 0, g->stream>>>(g->c, d_b, slot, kind, tol, max_iter, restart);
     CGCK(cudaGetLastError());
     g->h_sl[slot].state = H2GPU_CG_RUN;     // host view until the next sync
     return H2GPU_OK;
@@ -428,9 +445,7 @@ H2G_API int h2gpu_cg_step(h2gpu_cg* g, int n_iter)
         int st = h2gpu::image_apply_quiet(g->img, g->precision, width, g->c.P, kS, g->c.AP, kS);
         if (st != H2GPU_OK) return st;
         k_cg_dot<<<G, 256, 0, g->stream>>>(g->c);
-        k_cg_alpha<<<1, 256, 0, g->stream>>>(g->c);
         k_cg_update<<<G, 256, 0, g->stream>>>(g->c);
-        k_cg_finish<<<1, 256, 0, g->stream>>>(g->c);
     }
     CGCK(cudaGetLastError());
     CGCK(cudaEventRecord(g->done, g->stream));
@@ -447,7 +462,6 @@ H2G_API int h2gpu_cg_check(h2gpu_cg* g)
     int st = h2gpu::image_apply_quiet(g->img, H2GPU_PREC_FP64, width, g->c.X, kS, g->c.AP, kS);
     if (st != H2GPU_OK) return st;
     k_cg_resid<<<g->c.G, 256, 0, g->stream>>>(g->c);
-    k_cg_check_finish<<<1, 256, 0, g->stream>>>(g->c);
     CGCK(cudaGetLastError());
     CGCK(cudaEventRecord(g->done, g->stream));
     // a checked slot either finished or restarts: until the next sync the host view
@@ -510,9 +524,7 @@ H2G_API int h2gpu_cg_take(h2gpu_cg* g, int slot, double* d_x)
     if (g->h_sl[slot].state != H2GPU_CG_DONE)
         return h2gpu::set_error(H2GPU_ERR_STATE, "slot has no finished result (call h2gpu_cg_sync first)");
     CGCK(cudaSetDevice(g->device));
-    const size_t pitch = sizeof(double) * kS, col = sizeof(double);
-    CGCK(cudaMemcpy2DAsync(d_x, col, g->c.X + slot, pitch, col, g->N, cudaMemcpyDeviceToDevice, g->stream));
-    k_cg_free<<<1, 1, 0, g->stream>>>(g->d_sl, slot);
+    k_cg_take<<<std::max(1, std::min((g->N + 255) / 256, 148 * 8)), 256, 0, g->stream>>>(g->c, slot, d_x);
     CGCK(cudaGetLastError());
     CGCK(cudaStreamSynchronize(g->stream));
     g->h_sl[slot].state = H2GPU_CG_FREE;

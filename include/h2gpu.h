@@ -271,7 +271,7 @@ int h2gpu_set_jit_variant(h2gpu_image *img, int variant);
  * examples/SPDHSS-H2/pcg_tests.c:13-20, with FP64 vectors and inner products and
  * the operator in the image's precision at h2gpu_cg_create; a MATVEC slot computes
  * (K + mu I) b once.  All 16 slots are the columns of one panel, so each iteration
- * is one H2 matmul plus five small kernels, enqueued on the image's stream; the host
+ * is one H2 matmul plus three small kernels, enqueued on the image's stream; the host
  * reads the slot records with h2gpu_cg_sync once per batch of iterations.
  *
  * A slot whose recursive residual reaches tol ||b|| (or max_iter, or, for a mixed
