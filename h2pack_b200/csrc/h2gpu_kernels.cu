@@ -382,110 +382,155 @@ __device__ __forceinline__ void chunk_apply(const TA* __restrict__ A, int R, int
 
 // Stored blocks, single right-hand side (the matvec path, memory bound).  One launch.
 // A task of at most 256 columns, 512 rows and 128 KB (blk1_fits: the B blocks of the
-// usual leaf sizes, and their D blocks in FP32) is one warp's, 8 per CTA.  The lane owns
-// columns lane + 32j; their A^T w sums (and, for FP32 blocks, their inputs) live in the
-// warp's rows of shared memory for the whole block (only the lane touches its columns:
-// no barrier; registers stay free for the loads in flight).  The rows are walked 8
-// at a time with all of a pass's loads in flight (FP32: two 32-column passes, 16 loads
-// per lane), and the 8 rows' A v partials are combined with one transposed butterfly.
-// Every warp runs its own task, so 24 independent load chains per SM hide each other's
-// latency (one CTA per task left long serial chains of task, input, block loads,
-// barriers and output per ~100 KB block).  Larger tasks get a CTA each (blk1_cta): one
-// warp per 200 KB FP64 block measured slower (fewer warps than slots in the last
-// wave).  The plan orders each task list small-first; n_small is the count for TA.
-// Sums: FP64 blocks in FP64; FP32 blocks in FP32 over one pass (8 rows, or the <= 8
-// column passes of a row) and widened per sum.
-template <typename TA>
-__device__ __forceinline__ void blk1_warp(const BlkTask& T, const TA* __restrict__ arena,
+// usual leaf sizes, and their D blocks in FP32) is one warp's, 8 per CTA; every warp runs
+// its own task, so independent load chains hide each other's latency (one CTA per task
+// left long serial chains of task, input, block loads, barriers and output per ~100 KB
+// block).  Larger tasks get a CTA each (blk1_cta): one warp per 200 KB FP64 block measured
+// slower (fewer warps than slots in the last wave).  The plan orders each task list
+// small-first; n_small is the count for TA.
+//
+// A warp walks its rows eight at a time.  What bounds it is how many bytes a warp keeps on
+// their way.
+// FP64 (H2Pack's packing, rows on 8 bytes): the lane owns columns lane + 32 j, a pass of 32
+// columns at a time; their A^T w sums live in the warp's row of shared memory (only the lane
+// touches its columns: no barrier).  24 warps per SM; requesting the next pass during a pass
+// took registers from the warps and measured slower (B phase 0.61 -> 0.69 ms at N = 80,000).
+// FP32 (rows padded to 16 bytes): the lane owns four columns of each 128, 16 bytes a load,
+// both passes' sums and inputs in registers; a group's entries are requested while the group
+// before it is multiplied and reduced.  Coulomb N = 80,000, mixed: B phase 0.43 -> 0.33 ms, the
+// matvec 0.60 -> 0.49 ms against 4-byte loads in 24 warps per SM.
+// Sums: FP64 blocks in FP64; FP32 blocks in FP32 over eight rows, or a lane's eight entries
+// of a row, and widened per sum.
+__device__ __forceinline__ void blk1_warp(const BlkTask& T, const double* __restrict__ arena,
                                           const double* __restrict__ XS, double* __restrict__ PS,
-                                          double* __restrict__ sq, float* __restrict__ sv, int lane)
+                                          double* __restrict__ sq, int lane)
 {
-    constexpr bool F32 = sizeof(TA) == 4;
-    constexpr int PASS = F32 ? 2 : 1;          // 32-column passes whose loads are issued together
     const int ncol = T.ncol, nrow = T.nrow;
     const bool do0 = T.out0_row >= 0, do1 = T.out1_row >= 0;
     const int J = (ncol + 31) >> 5;
-    const TA* A = arena + blk_off<TA>(T);
-    const int lda = blk_ld<TA>(T);
+    const double* A = arena + T.a_off;
 #pragma unroll
-    for (int j = 0; j < 8; j++)
-    {
-        const int c = lane + 32 * j;
-        sq[c] = 0.0;
-        if constexpr (F32) sv[c] = (do0 && c < ncol) ? (float) XS[T.in0_row + c] : 0.f;
-    }
+    for (int j = 0; j < 8; j++) sq[lane + 32 * j] = 0.0;
     for (int r0 = 0; r0 < nrow; r0 += 8)
     {
         const int nr = min(8, nrow - r0);
-        double wr[8];
+        double wr[8], p[8];
 #pragma unroll
         for (int k = 0; k < 8; k++) wr[k] = (do1 && k < nr) ? XS[T.in1_row + r0 + k] : 0.0;
-        double p[8];
-        float pf[8];
 #pragma unroll
-        for (int k = 0; k < 8; k++) { p[k] = 0.0; pf[k] = 0.f; }
+        for (int k = 0; k < 8; k++) p[k] = 0.0;
 #pragma unroll 1
-        for (int j0 = 0; j0 < J; j0 += PASS)
+        for (int j = 0; j < J; j++)
         {
-            TA a[PASS][8];
+            const int c = lane + 32 * j;
+            const bool cv = c < ncol;
+            double a[8];
 #pragma unroll
-            for (int u = 0; u < PASS; u++)
+            for (int k = 0; k < 8; k++) a[k] = (cv && k < nr) ? A[(long long) (r0 + k) * ncol + c] : 0.0;
+            const double v = (do0 && cv) ? XS[T.in0_row + c] : 0.0;
+            double q = 0.0;
+#pragma unroll
+            for (int k = 0; k < 8; k++)
             {
-                const int c = lane + 32 * (j0 + u);
-                const bool cv = c < ncol;
-#pragma unroll
-                for (int k = 0; k < 8; k++) a[u][k] = (cv && k < nr) ? A[(long long) (r0 + k) * lda + c] : TA(0);
+                q = fma(a[k], wr[k], q);
+                p[k] = fma(a[k], v, p[k]);
             }
-#pragma unroll
-            for (int u = 0; u < PASS; u++)
-            {
-                const int j = j0 + u;
-                if constexpr (F32)
-                {
-                    const float v = sv[lane + 32 * j];
-                    float q = 0.f;
-#pragma unroll
-                    for (int k = 0; k < 8; k++)
-                    {
-                        q = fmaf(a[u][k], (float) wr[k], q);
-                        pf[k] = fmaf(a[u][k], v, pf[k]);
-                    }
-                    sq[lane + 32 * j] += (double) q;
-                } else {
-                    const int c = lane + 32 * j;
-                    const double v = (do0 && c < ncol) ? XS[T.in0_row + c] : 0.0;
-                    double q = 0.0;
-#pragma unroll
-                    for (int k = 0; k < 8; k++)
-                    {
-                        q = fma(to_d(a[u][k]), wr[k], q);
-                        p[k] = fma(to_d(a[u][k]), v, p[k]);
-                    }
-                    sq[lane + 32 * j] += q;
-                }
-            }
+            sq[c] += q;
         }
         if (do0)
         {
-            if constexpr (F32)
-            {
-#pragma unroll
-                for (int k = 0; k < 8; k++) p[k] = (double) pf[k];
-            }
             warp_transpose_reduce<8>(p, lane);
             const int row = nv_of_lane<8>(lane);
             if (lane_writes<8>(lane) && row < nr) PS[T.out0_row + r0 + row] = p[0];
         }
     }
     if (do1)
-    {
 #pragma unroll
         for (int j = 0; j < 8; j++)
+            if (lane + 32 * j < ncol) PS[T.out1_row + lane + 32 * j] = sq[lane + 32 * j];
+}
+
+__device__ __forceinline__ void blk1_warp(const BlkTask& T, const float* __restrict__ arena,
+                                          const double* __restrict__ XS, double* __restrict__ PS, double*, int lane)
+{
+    const int ncol = T.ncol, nrow = T.nrow, ld = T.ld32;
+    const bool do0 = T.out0_row >= 0, do1 = T.out1_row >= 0;
+    const float* A = arena + T.a32;
+    // passes 0 and 1: columns 4 lane .. + 3 and 128 more (past the padded row: nothing)
+    float v[2][4];
+    double q[2][4];
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+#pragma unroll
+        for (int h = 0; h < 4; h++)
         {
-            const int c = lane + 32 * j;
-            if (c < ncol) PS[T.out1_row + c] = sq[c];
+            const int c = 128 * u + 4 * lane + h;
+            v[u][h] = (do0 && c < ncol) ? (float) XS[T.in0_row + c] : 0.f;
+            q[u][h] = 0.0;
+        }
+    const bool in0 = 4 * lane < ld, in1 = 128 + 4 * lane < ld, two = ncol > 128;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto fetch = [&](int r0, int u, float4 (&a)[8]) {
+        const bool in = u ? in1 : in0;
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            a[k] = (in && r0 + k < nrow)
+                       ? __ldg(reinterpret_cast<const float4*>(A + (long long) (r0 + k) * ld + 128 * u + 4 * lane)) : zero;
+    };
+    auto use = [&](const float4 (&a)[8], int u, const float (&w)[8], float (&p)[8]) {
+        float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+        {
+            s0 = fmaf(a[k].x, w[k], s0);
+            s1 = fmaf(a[k].y, w[k], s1);
+            s2 = fmaf(a[k].z, w[k], s2);
+            s3 = fmaf(a[k].w, w[k], s3);
+            p[k] = fmaf(a[k].x, v[u][0], p[k]);
+            p[k] = fmaf(a[k].y, v[u][1], p[k]);
+            p[k] = fmaf(a[k].z, v[u][2], p[k]);
+            p[k] = fmaf(a[k].w, v[u][3], p[k]);
+        }
+        q[u][0] += (double) s0;
+        q[u][1] += (double) s1;
+        q[u][2] += (double) s2;
+        q[u][3] += (double) s3;
+    };
+    float4 a0[8], a1[8];
+    fetch(0, 0, a0);
+    if (two) fetch(0, 1, a1);
+#pragma unroll 1
+    for (int r0 = 0; r0 < nrow; r0 += 8)
+    {
+        const int nr = min(8, nrow - r0);
+        float w[8], pf[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) w[k] = (do1 && k < nr) ? (float) XS[T.in1_row + r0 + k] : 0.f;
+#pragma unroll
+        for (int k = 0; k < 8; k++) pf[k] = 0.f;
+        use(a0, 0, w, pf);
+        if (r0 + 8 < nrow) fetch(r0 + 8, 0, a0);
+        if (two)
+        {
+            use(a1, 1, w, pf);
+            if (r0 + 8 < nrow) fetch(r0 + 8, 1, a1);
+        }
+        if (do0)
+        {
+            double p[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) p[k] = (double) pf[k];
+            warp_transpose_reduce<8>(p, lane);
+            const int row = nv_of_lane<8>(lane);
+            if (lane_writes<8>(lane) && row < nr) PS[T.out0_row + r0 + row] = p[0];
         }
     }
+    if (do1)
+#pragma unroll
+        for (int u = 0; u < 2; u++)
+#pragma unroll
+            for (int h = 0; h < 4; h++)
+                if (128 * u + 4 * lane + h < ncol) PS[T.out1_row + 128 * u + 4 * lane + h] = q[u][h];
 }
 
 // A task walked by the whole CTA (chunks of 64 rows; warp w owns rows 8w..8w+7 of a
@@ -599,12 +644,11 @@ __device__ __forceinline__ void blk1_cta(const BlkTask& T, const TA* __restrict_
 // CTAs [0, ceil(n_small / 8)): 8 small tasks each, one per warp; the rest: one larger
 // task each (tasks [n_small, n)).
 template <typename TA>
-__global__ void __launch_bounds__(256, 3) k_blk1(const BlkTask* __restrict__ tasks, int n, int n_small,
+__global__ void __launch_bounds__(256, sizeof(TA) == 4 ? 2 : 3) k_blk1(const BlkTask* __restrict__ tasks, int n, int n_small,
                                               const TA* __restrict__ arena, const double* __restrict__ XS,
                                               double* __restrict__ PS)
 {
     __shared__ double s_q[kWarps][256];
-    __shared__ float s_v[sizeof(TA) == 4 ? kWarps : 1][256];
     const int nw = (n_small + kWarps - 1) / kWarps;
     if ((int) blockIdx.x < nw)
     {
@@ -613,7 +657,7 @@ __global__ void __launch_bounds__(256, 3) k_blk1(const BlkTask* __restrict__ tas
         if (t < n_small)
         {
             const BlkTask T = tasks[t];
-            blk1_warp<TA>(T, arena, XS, PS, s_q[w], s_v[sizeof(TA) == 4 ? w : 0], threadIdx.x & 31);
+            blk1_warp(T, arena, XS, PS, s_q[w], threadIdx.x & 31);
         }
         return;
     }
