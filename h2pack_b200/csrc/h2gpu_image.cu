@@ -592,8 +592,8 @@ int build_plan(h2gpu_image* im, const h2gpu_desc* d, HostPlan& hp)
             im->blk1_small[li][0] = n64;
             im->blk1_small[li][1] = n32;
         }
-        // units of the 64-wide passes: pass 0 per 64-row chunk of a task (A V), pass 1 per
-        // 64-column tile of a task (A^T W)
+        // units of the 64-wide passes: pass 0 per 128-row chunk of a task (A V), pass 1 per
+        // 128-column tile of a task (A^T W)
         // Pass-0 units are ordered by their input rows (the column node's y0 / x slice),
         // so that consecutive units, walked by the persistent CTAs in order, read the same
         // 64-wide input rows from L2; pass-1 units read their task's own rows and keep the
@@ -604,7 +604,7 @@ int build_plan(h2gpu_image* im, const h2gpu_desc* d, HostPlan& hp)
             {
                 const BlkTask& t = ts[i];
                 if ((pass == 0 ? t.out0_row : t.out1_row) < 0) continue;
-                for (int o = 0; o < (pass == 0 ? t.nrow : t.ncol); o += 64) us.push_back(WideUnit{i, o});
+                for (int o = 0; o < (pass == 0 ? t.nrow : t.ncol); o += kWideRows) us.push_back(WideUnit{i, o});
             }
             if (pass == 0)
                 std::stable_sort(us.begin(), us.end(), [&](const WideUnit& a, const WideUnit& b) {
@@ -1354,7 +1354,7 @@ int check_plan(const h2gpu_image* im, const h2gpu_desc* d, const HostPlan& hp, l
         };
         TRY(cover_blocks("B", hp.blkB, d->n_B, d->B_nrow, d->B_ncol, d->B_ptr));
         TRY(cover_blocks("D", hp.blkD, d->n_D, d->D_nrow, d->D_ncol, d->D_ptr));
-        // ---- units of the 64-wide passes: every 64-row chunk (pass 0) and every 64-column
+        // ---- units of the 64-wide passes: every 128-row chunk (pass 0) and every 128-column
         //      tile (pass 1) of every task that has the product, once each
         long long w0 = 0;
         const int* nw = im->n_wide;
@@ -1371,9 +1371,9 @@ int check_plan(const h2gpu_image* im, const h2gpu_desc* d, const HostPlan& hp, l
                 const BlkTask& t = ts[u.task];
                 const int ext = pass == 0 ? t.nrow : t.ncol;
                 REQ((pass == 0 ? t.out0_row : t.out1_row) >= 0, "plan: a wide unit of a product its task lacks");
-                REQ(u.off >= 0 && u.off < ext && u.off % 64 == 0, "plan: a wide unit starts off its 64-grid");
-                if (seen[u.task].empty()) seen[u.task].assign((ext + 63) / 64, 0);
-                REQ(++seen[u.task][u.off / 64] == 1, "plan: a wide unit repeats");
+                REQ(u.off >= 0 && u.off < ext && u.off % kWideRows == 0, "plan: a wide unit starts off its grid");
+                if (seen[u.task].empty()) seen[u.task].assign((ext + kWideRows - 1) / kWideRows, 0);
+                REQ(++seen[u.task][u.off / kWideRows] == 1, "plan: a wide unit repeats");
             }
             for (size_t i = 0; i < ts.size(); i++)
                 if ((pass == 0 ? ts[i].out0_row : ts[i].out1_row) >= 0)

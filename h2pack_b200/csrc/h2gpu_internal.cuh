@@ -80,9 +80,10 @@ __host__ __device__ inline bool blk1_fits(int nrow, int ncol, int elem_bytes)
     return ncol <= kBlk1WarpCols && nrow <= kBlk1WarpRows && (long long) nrow * ncol * elem_bytes <= kBlk1WarpBytes;
 }
 
-// Unit of the wide-panel stored-block passes: one 64-row chunk of a task (pass 0,
-// A V over all column tiles) or one 64-column tile of a task (pass 1, A^T W over all of
+// Unit of the wide-panel stored-block passes: one 128-row chunk of a task (pass 0,
+// A V over all column tiles) or one 128-column tile of a task (pass 1, A^T W over all of
 // the task's rows).
+constexpr int kWideRows = 128;
 struct WideUnit {
     int task;          // index into the block-task list
     int off;           // first row (pass 0) or first column (pass 1) of the unit

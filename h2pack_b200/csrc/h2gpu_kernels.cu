@@ -3016,33 +3016,39 @@ __global__ void __launch_bounds__(kBf3Threads, 2) k_blk_bf3w(const BlkTask* __re
 
 // ------------------------ stored blocks on tcgen05, 64-wide panels as two GEMM passes
 
-// Instruction descriptor, kind::f16 with BF16 A and B, FP32 accumulator, M = 64, N = n,
+// Instruction descriptor, kind::f16 with BF16 A and B, FP32 accumulator, M = 128, N = n,
 // A and B each K-major (0) or MN-major (1).
 __host__ __device__ constexpr uint32_t umma_idesc_bf16_ab(int n, int a_mn_major, int b_mn_major)
 {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t) a_mn_major << 15) | ((uint32_t) b_mn_major << 16) |
-           ((uint32_t) (n >> 3) << 17) | ((uint32_t) (64 >> 4) << 24);
+           ((uint32_t) (n >> 3) << 17) | ((uint32_t) (128 >> 4) << 24);
 }
 
 // A panel of 64 right-hand sides applied to the stored blocks as two passes over the block
 // tasks, each a plain GEMM whose outputs are written once (the one-pass kernel's per-tile
 // read-modify-write of the transposed-product slot dominated its memory traffic):
-//   pass 0, one unit per 64-row chunk of a task:     C0 = A_chunk V    (over the column tiles)
-//   pass 1, one unit per 64-column tile of a task:   C1 = A_tile^T W   (over the task's rows)
-// Each 64 x 64 tile of A (FP32) is split into BF16 pieces h + m + l in shared memory
-// (rows of 128 B, 128-byte swizzle).  The right-hand sides of a tile (64 rows of the
-// input space, row-major with the 64 right-hand sides contiguous) are split the same way
-// and used as an MN-major B operand, so they are read with coalesced loads and need no
-// transpose.  Six products per 16-deep K step (l.h + h.l + m.m + m.h + h.m + h.h), FP32 in
-// TMEM over one tile (64 terms), FP64 across tiles in shared memory; the unit's 64 output
-// rows are written once.  The next tile is loaded into registers while the MMAs of the
-// current one run.  Bounded waits record a status and stop.
+//   pass 0, one unit per 128-row chunk of a task:     C0 = A_chunk V    (over the column tiles)
+//   pass 1, one unit per 128-column tile of a task:   C1 = A_tile^T W   (over the task's rows)
+// A unit is walked in tiles of 64 along the summed dimension.  Each 128 x 64 (64 x 128) tile
+// of A (FP32) is split into BF16 pieces h + m + l in shared memory (128-byte rows, 128-byte
+// swizzle).  The right-hand sides of a tile (64 rows of the input space, row-major with the
+// 64 right-hand sides contiguous) come split by k_split3 and are an MN-major B operand, so
+// they are copied as they are.  Six products per 16-deep K step (l.h + h.l + m.m + m.h + h.m
+// + h.h), FP32 in TMEM over one tile (64 terms), FP64 across tiles in registers.
+//
+// What bounds it: blocks of 100 to 400 rows and columns are one to four tiles per unit, so
+// any step that waits for the step before it is exposed once or twice a unit (64-row units
+// with all threads taking the steps in turn: 5.7 us per 16 KB tile).  The roles are separate
+// warps that run ahead of each other through two stages, across units: 8 warps load A
+// (one tile ahead, in registers) and split it, one thread issues the MMAs, 8 warps read the
+// products and sum.  RPY N = 20,011, 64 right-hand sides: the two passes over B 6.0 -> 3.7 ms,
+// the matmul 8.3 -> 5.05.  Bounded waits record a status and stop.
 struct WideSmem {
-    uint16_t a[3][64 * 64];    // A tile pieces: 64 rows (of A) of 64 BF16, 128-byte swizzle
-    uint16_t b[2][3][64 * 64]; // right-hand-side pieces, two stages: 64 rows (k) of 64 BF16, swizzled
-    double acc[64][65];        // FP64 sums of the unit's 64 output rows (padded)
-    unsigned long long mbar;
+    uint16_t a[2][3][128 * 64];   // two stages of A tile pieces
+    uint16_t b[2][3][64 * 64];    // two stages of right-hand-side pieces: 64 rows (k) of 64 BF16
+    unsigned long long full[2], empty[2], tfull[2], tempty[2];   // mbarriers: operands, accumulators
     uint32_t tmem;
+    int abort;                    // a wait ran out: every role stops
 };
 
 constexpr int wide_smem_bytes() { return (int) sizeof(WideSmem) + 1024; }
@@ -3062,7 +3068,7 @@ __device__ __forceinline__ void bf16x3_pair(float x0, float x1, uint32_t& h, uin
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(l) : "f"(r2.y), "f"(r2.x));
 }
 
-constexpr int kWideThreads = 256;
+constexpr int kWideThreads = 32 * 17;   // 8 warps load, 8 warps sum, 1 issues the MMAs
 
 // 16-byte global -> shared copy whose bytes past src_bytes (0 or 16) are zero-filled
 __device__ __forceinline__ void cp_async16_zfill(void* dst, const void* src, int src_bytes)
@@ -3094,204 +3100,255 @@ __global__ void k_split3(const double* __restrict__ XS, long long row0, long lon
     }
 }
 
+// One unit of a pass, and its walk by a persistent CTA: units blockIdx.x, + gridDim.x, ..
 template <int MODE>
-__global__ void __launch_bounds__(kWideThreads, 2) k_blk_wide(const BlkTask* __restrict__ tasks,
+struct WideWalk {
+    const BlkTask* tasks;
+    const WideUnit* units;
+    int n, ui;          // units; the current one
+    BlkTask T, Tn;      // its task; the next unit's, read one unit ahead
+    int off, offn, nt;  // first row (column) of the unit; its tiles
+    __device__ __forceinline__ void read_next()
+    {
+        if (ui + (int) gridDim.x < n)
+        {
+            const WideUnit U = units[ui + gridDim.x];
+            Tn = tasks[U.task];
+            offn = U.off;
+        }
+    }
+    __device__ __forceinline__ void take()
+    {
+        T = Tn;
+        off = offn;
+        nt = ((MODE == 0 ? T.ncol : T.nrow) + 63) / 64;
+        read_next();
+    }
+    __device__ __forceinline__ bool begin(const BlkTask* t, const WideUnit* u, int count)
+    {
+        tasks = t; units = u; n = count;
+        ui = (int) blockIdx.x - (int) gridDim.x;
+        if ((int) blockIdx.x >= n) return false;
+        read_next();
+        ui += gridDim.x;
+        take();
+        return true;
+    }
+    __device__ __forceinline__ bool next()
+    {
+        ui += gridDim.x;
+        if (ui >= n) return false;
+        take();
+        return true;
+    }
+    // rows (pass 0) or columns (pass 1) of the unit
+    __device__ __forceinline__ int extent() const { return min(128, (MODE == 0 ? T.nrow : T.ncol) - off); }
+};
+
+template <int MODE>
+__global__ void __launch_bounds__(kWideThreads, 1) k_blk_wide(const BlkTask* __restrict__ tasks,
                                                               const WideUnit* __restrict__ units, int n_units,
                                                               const float* __restrict__ arena,
                                                               const uint16_t* __restrict__ XS3, long long rows3,
                                                               double* __restrict__ PS, int* __restrict__ status)
 {
-    constexpr int NV = 64;
+    constexpr int NV = 64, NL = 256;              // right-hand sides; loading (and summing) threads
     // pass 0: A K-major, B (V rows) MN-major; pass 1: A MN-major (A^T), B (W rows) MN-major
     constexpr uint32_t IDESC = umma_idesc_bf16_ab(NV, MODE == 1 ? 1 : 0, 1);
-    constexpr int STAGE_B = 3 * 64 * 64 * 2;      // bytes of one stage of right-hand-side pieces
+    constexpr int PIECE_A = 128 * 64 * 2, STAGE_A = 3 * PIECE_A, PIECE_B = 64 * 64 * 2, STAGE_B = 3 * PIECE_B;
     extern __shared__ __align__(1024) unsigned char wide_raw[];
     WideSmem& sm = *reinterpret_cast<WideSmem*>(wide_raw + ((1024 - (smem_u32(wide_raw) & 1023)) & 1023));
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-
-    if (warp == 0)
+    if (warp == 16)
     {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 64;" ::"r"(smem_u32(&sm.tmem)) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 128;" ::"r"(smem_u32(&sm.tmem)) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid == 0)
     {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&sm.mbar)) : "memory");
+        sm.abort = 0;
+        for (int k = 0; k < 2; k++)
+        {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&sm.full[k])), "r"(NL) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&sm.empty[k])) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&sm.tfull[k])) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&sm.tempty[k])), "r"(NL) : "memory");
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = sm.tmem, mbar = smem_u32(&sm.mbar);
+    const uint32_t tmem = sm.tmem;
     unsigned char* const a_b = reinterpret_cast<unsigned char*>(sm.a);
     unsigned char* const b_b = reinterpret_cast<unsigned char*>(sm.b);
-    const uint32_t a_s = smem_u32(sm.a), b_s = smem_u32(sm.b);
-    bool ok = true;
-    uint32_t phase = 0;
-    // warp w reads TMEM lane quadrant w % 4 (rows 16 (w % 4) + lane, lane < 16) and the 32
-    // accumulator columns 32 (w / 4) .. + 31
-    const int quad = warp & 3, half = warp >> 2;
-    double* const acc = sm.acc[(16 * quad + lane) & 63] + 32 * half;
-    constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};
-
-    // persistent: the CTA takes units blockIdx.x, + gridDim.x, ...
-    for (int ui = blockIdx.x; ui < n_units && ok; ui += gridDim.x)
-    {
-        const WideUnit U = units[ui];
-        const BlkTask T = tasks[U.task];
-        const int ncol = T.ncol, nrow = T.nrow;
-        // the unit's fixed 64-row chunk (pass 0) or 64-column tile (pass 1), and the tiles it walks
-        const int nt = MODE == 0 ? (ncol + 63) / 64 : (nrow + 63) / 64;
-        const float* A0 = arena + T.a32;
-        const int lda = T.ld32;
-        auto tile_of = [&](int t, int& rc, int& c0) {
-            if (MODE == 0) { rc = U.off; c0 = 64 * t; }
-            else { rc = 64 * t; c0 = U.off; }
-        };
-        // the A tile is loaded into registers (thread t: 2 granules, row r, 8 consecutive
-        // columns q, as two 16-byte loads: FP32 rows are padded to 16 bytes with zeros, so
-        // a vector that starts before the row's end stays in the row) and split into shared
-        // memory; the right-hand-side pieces of a tile are copied from XS3 by cp.async into
-        // one of two stages (rows past the tile's extent zero-filled)
-        float4 ra[2][2];
-        auto load_a = [&](int t) {
-            int rc, c0;
-            tile_of(t, rc, c0);
-            const int R = min(64, nrow - rc), C = min(64, ncol - c0);
-            const float* A = A0 + (long long) rc * lda + c0;
-#pragma unroll
-            for (int u = 0; u < 2; u++)
+    auto wait = [&](unsigned long long* bar, int parity) {
+        volatile int* const ab = &sm.abort;
+        for (int it = 1; !mbar_try_wait(smem_u32(bar), (uint32_t) parity); it++)
+            if ((it & 255) == 0 && (*ab || it > (1 << 22)))
             {
-                const int gi = tid + kWideThreads * u, r = gi >> 3, q = gi & 7;
+                *ab = 1;
+                atomicExch(status, 1);
+                return false;
+            }
+        return true;
+    };
+    auto arrive = [&](unsigned long long* bar) {
+        asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.shared::cta.b64 t, [%0];\n\t}" ::"r"(smem_u32(bar)) : "memory");
+    };
+    WideWalk<MODE> w;
+    if (warp < 8)
+    {
+        // ---- loaders.  A: four granules of 8 consecutive values of a row per thread, as two
+        // 16-byte loads each (FP32 rows are padded to 16 bytes with zeros, so a vector that
+        // starts before the row's end stays in the row); zeros outside the unit.
+        float4 ra[4][2];
+        auto load_a = [&](int t) {
+            const int M = w.extent(), K = min(64, (MODE == 0 ? w.T.ncol : w.T.nrow) - 64 * t), ld = w.T.ld32;
+            const float* A = arena + w.T.a32 + (MODE == 0 ? (long long) w.off * ld + 64 * t : (long long) (64 * t) * ld + w.off);
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+            {
+                const int gi = tid + NL * u;
+                const int r = MODE == 0 ? gi >> 3 : gi >> 4, c = 8 * (MODE == 0 ? gi & 7 : gi & 15);
 #pragma unroll
                 for (int h = 0; h < 2; h++)
-                {
-                    const int c = 8 * q + 4 * h;
-                    ra[u][h] = (r < R && c < C) ? *reinterpret_cast<const float4*>(A + (long long) r * lda + c)
-                                                : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
+                    ra[u][h] = (MODE == 0 ? r < M && c + 4 * h < K : r < K && c + 4 * h < M)
+                                   ? __ldg(reinterpret_cast<const float4*>(A + (long long) r * ld + c + 4 * h))
+                                   : make_float4(0.f, 0.f, 0.f, 0.f);
             }
         };
-        auto issue_b = [&](int t, int stage) {
-            int rc, c0;
-            tile_of(t, rc, c0);
-            const int nk = MODE == 0 ? min(64, ncol - c0) : min(64, nrow - rc);
-            const long long row0 = MODE == 0 ? (long long) T.in0_row + c0 : (long long) T.in1_row + rc;
+        auto store_a = [&](int st) {
 #pragma unroll
-            for (int u = 0; u < 6; u++)
+            for (int u = 0; u < 4; u++)
             {
-                const int i = tid + kWideThreads * u, pc = i >> 9, r = (i >> 3) & 63, q = i & 7;
-                const uint16_t* src = XS3 + ((long long) pc * rows3 + row0 + (r < nk ? r : 0)) * 64 + 8 * q;
-                cp_async16_zfill(b_b + stage * STAGE_B + pc * 8192 + sw128(r, q), src, r < nk ? 16 : 0);
-            }
-            cp_async_commit();
-        };
-        auto store_a = [&]() {
-#pragma unroll
-            for (int u = 0; u < 2; u++)
-            {
-                const int gi = tid + kWideThreads * u, r = gi >> 3, q = gi & 7;
+                const int gi = tid + NL * u;
                 uint32_t h[4], m[4], l[4];
                 bf16x3_pair(ra[u][0].x, ra[u][0].y, h[0], m[0], l[0]);
                 bf16x3_pair(ra[u][0].z, ra[u][0].w, h[1], m[1], l[1]);
                 bf16x3_pair(ra[u][1].x, ra[u][1].y, h[2], m[2], l[2]);
                 bf16x3_pair(ra[u][1].z, ra[u][1].w, h[3], m[3], l[3]);
-                const int off = sw128(r, q);
+                // pass 0: 128 rows of 64; pass 1: two column halves of 64 rows of 64
+                const int off = st * STAGE_A + (MODE == 0 ? sw128(gi >> 3, gi & 7) : ((gi >> 3) & 1) * 8192 + sw128(gi >> 4, gi & 7));
                 *reinterpret_cast<uint4*>(a_b + off) = make_uint4(h[0], h[1], h[2], h[3]);
-                *reinterpret_cast<uint4*>(a_b + 8192 + off) = make_uint4(m[0], m[1], m[2], m[3]);
-                *reinterpret_cast<uint4*>(a_b + 16384 + off) = make_uint4(l[0], l[1], l[2], l[3]);
+                *reinterpret_cast<uint4*>(a_b + PIECE_A + off) = make_uint4(m[0], m[1], m[2], m[3]);
+                *reinterpret_cast<uint4*>(a_b + 2 * PIECE_A + off) = make_uint4(l[0], l[1], l[2], l[3]);
             }
         };
-        // wait for the tile's MMAs and add its FP32 products into the unit's FP64 sums (the
-        // unit's first tile initialises them)
-        auto drain = [&](bool first) {
-            int good = 1;
-            if (tid == 0)
-            {
-                int it = 0;
-                while (!mbar_try_wait(mbar, phase))
-                    if (++it > (1 << 22)) { good = 0; break; }
-                if (!good) atomicExch(status, 1);
-            }
-            phase ^= 1;
-            ok = __syncthreads_and(good) != 0;
-            if (!ok) return;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            uint32_t d[32];
-            asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-                         "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-                         : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]),
-                           "=r"(d[8]), "=r"(d[9]), "=r"(d[10]), "=r"(d[11]), "=r"(d[12]), "=r"(d[13]), "=r"(d[14]), "=r"(d[15]),
-                           "=r"(d[16]), "=r"(d[17]), "=r"(d[18]), "=r"(d[19]), "=r"(d[20]), "=r"(d[21]), "=r"(d[22]), "=r"(d[23]),
-                           "=r"(d[24]), "=r"(d[25]), "=r"(d[26]), "=r"(d[27]), "=r"(d[28]), "=r"(d[29]), "=r"(d[30]), "=r"(d[31])
-                         : "r"(tmem + ((uint32_t) (32 * quad) << 16) + (uint32_t) (32 * half)));
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (lane < 16)
-            {
-                if (first)
-#pragma unroll
-                    for (int n = 0; n < 32; n++) acc[n] = (double) __uint_as_float(d[n]);
-                else
-#pragma unroll
-                    for (int n = 0; n < 32; n++) acc[n] += (double) __uint_as_float(d[n]);
-            }
-        };
-
-        issue_b(0, 0);
-        load_a(0);
-        for (int t = 0; t < nt; t++)
+        bool more = w.begin(tasks, units, n_units);
+        if (more) load_a(0);
+        for (int i = 0, t = 0; more; i++)
         {
-            if (t > 0) drain(t == 1);
-            if (!ok) break;
-            store_a();
-            cp_async_wait_all();                     // this thread's copies of tile t's inputs
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncthreads();
-            if (tid == 0)
+            const int st = i & 1;
+            if (i >= 2 && !wait(&sm.empty[st], ((i >> 1) - 1) & 1)) break;
+            const int nk = min(64, (MODE == 0 ? w.T.ncol : w.T.nrow) - 64 * t);
+            const long long row0 = (long long) (MODE == 0 ? w.T.in0_row : w.T.in1_row) + 64 * t;
+#pragma unroll
+            for (int u = 0; u < 6; u++)
             {
+                const int e = tid + NL * u, pc = e >> 9, r = (e >> 3) & 63, q = e & 7;
+                const uint16_t* src = XS3 + ((long long) pc * rows3 + row0 + (r < nk ? r : 0)) * 64 + 8 * q;
+                cp_async16_zfill(b_b + st * STAGE_B + pc * PIECE_B + sw128(r, q), src, r < nk ? 16 : 0);
+            }
+            cp_async_commit();
+            store_a(st);
+            if (++t == w.nt)
+            {
+                t = 0;
+                more = w.next();
+            }
+            if (more) load_a(t);                 // in flight until the next tile's split
+            cp_async_wait_all();
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            arrive(&sm.full[st]);
+        }
+        cp_async_wait_all();
+    }
+    else if (warp < 16)
+    {
+        // ---- sums: a thread owns row 32 (warp % 4) + lane of the unit and 32 right-hand sides
+        const int quad = warp & 3, half = (warp - 8) >> 2;
+        double acc[32];
+        int i = 0;
+        for (bool more = w.begin(tasks, units, n_units); more; more = w.next())
+        {
+            bool ok = true;
+            for (int t = 0; t < w.nt; t++, i++)
+            {
+                const int d = i & 1;
+                if (!(ok = __all_sync(kFull, wait(&sm.tfull[d], (i >> 1) & 1)))) break;   // the loads below are the warp's
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t bs = b_s + (uint32_t) ((t & 1) * STAGE_B);
+#pragma unroll
+                for (int g = 0; g < 2; g++)
+                {
+                    uint32_t x[16];
+                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,"
+                                 "%15}, [%16];"
+                                 : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]), "=r"(x[4]), "=r"(x[5]), "=r"(x[6]), "=r"(x[7]),
+                                   "=r"(x[8]), "=r"(x[9]), "=r"(x[10]), "=r"(x[11]), "=r"(x[12]), "=r"(x[13]), "=r"(x[14]), "=r"(x[15])
+                                 : "r"(tmem + ((uint32_t) (32 * quad) << 16) + (uint32_t) (64 * d + 32 * half + 16 * g)));
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (g == 1)
+                    {
+                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                        arrive(&sm.tempty[d]);
+                    }
+#pragma unroll
+                    for (int n = 0; n < 16; n++)
+                        acc[16 * g + n] = (t == 0 ? 0.0 : acc[16 * g + n]) + (double) __uint_as_float(x[n]);
+                }
+            }
+            if (!ok) break;
+            const int m = 32 * quad + lane;
+            if (m < w.extent())
+            {
+                // 16 bytes a store: rows of 64 doubles, 32 of them this thread's
+                double2* o = reinterpret_cast<double2*>(PS + (long long) ((MODE == 0 ? w.T.out0_row : w.T.out1_row) + w.off + m) * NV + 32 * half);
+#pragma unroll
+                for (int n = 0; n < 16; n++) o[n] = make_double2(acc[2 * n], acc[2 * n + 1]);
+            }
+        }
+    }
+    else if (lane == 0)
+    {
+        // ---- MMA issue
+        constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};
+        int i = 0;
+        bool ok = true;
+        for (bool more = w.begin(tasks, units, n_units); more && ok; more = w.next())
+            for (int t = 0; t < w.nt; t++, i++)
+            {
+                const int st = i & 1;
+                if (!(ok = wait(&sm.full[st], (i >> 1) & 1))) break;
+                if (i >= 2 && !(ok = wait(&sm.tempty[st], ((i >> 1) - 1) & 1))) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t as = smem_u32(sm.a) + (uint32_t) (st * STAGE_A), bs = smem_u32(sm.b) + (uint32_t) (st * STAGE_B);
 #pragma unroll
                 for (int ks = 0; ks < 4; ks++)          // K-steps of 16
 #pragma unroll
                     for (int p = 0; p < 6; p++)
                     {
-                        // pass 0: A K-major (32-byte step along a row); pass 1: A MN-major
-                        // (16 rows = two 8-row swizzle atoms per step); B MN-major in both
-                        const uint64_t ad = MODE == 0 ? umma_desc(a_s + PA[p] * 8192 + ks * 32, 16, 1024, 2)
-                                                      : umma_desc(a_s + PA[p] * 8192 + ks * 2048, 8192, 1024, 2);
-                        umma_f16(tmem, ad, umma_desc(bs + PB[p] * 8192 + ks * 2048, 8192, 1024, 2), IDESC,
+                        // pass 0: A K-major (32-byte step along a row); pass 1: A MN-major (16
+                        // rows = two 8-row swizzle atoms per step, the second 64 columns 8 KB
+                        // on); B MN-major in both
+                        const uint64_t ad = MODE == 0 ? umma_desc(as + PA[p] * PIECE_A + ks * 32, 16, 1024, 2)
+                                                      : umma_desc(as + PA[p] * PIECE_A + ks * 2048, 8192, 1024, 2);
+                        umma_f16(tmem + (uint32_t) (64 * st), ad, umma_desc(bs + PB[p] * PIECE_B + ks * 2048, 8192, 1024, 2), IDESC,
                                  (ks == 0 && p == 0) ? 0u : 1u);
                     }
-                umma_commit(mbar);
+                umma_commit(smem_u32(&sm.empty[st]));
+                umma_commit(smem_u32(&sm.tfull[st]));
             }
-            if (t + 1 < nt)
-            {
-                issue_b(t + 1, (t + 1) & 1);         // that stage's previous tile (t - 1) was waited on
-                load_a(t + 1);
-            }
-        }
-        if (ok && nt > 0) drain(nt == 1);
-        // the unit's outputs, written once (each thread writes the sums it added)
-        if (ok && lane < 16)
-        {
-            const int m = 16 * quad + lane;
-            const int lim = MODE == 0 ? min(64, nrow - U.off) : min(64, ncol - U.off);
-            if (m < lim)
-            {
-                double* o = PS + (long long) ((MODE == 0 ? T.out0_row : T.out1_row) + U.off + m) * NV + 32 * half;
-#pragma unroll 8
-                for (int n = 0; n < 32; n++) o[n] = acc[n];
-            }
-        }
+        // the last MMAs have completed before the tensor memory is given back
+        for (int k = max(0, i - 2); k < i; k++) wait(&sm.tfull[k & 1], (k >> 1) & 1);
     }
+    __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 0)
+    if (warp == 16)
     {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 64;" ::"r"(tmem) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 128;" ::"r"(tmem) : "memory");
     }
 }
 
@@ -4108,7 +4165,7 @@ cudaError_t launch_blk_wide(int mode, const BlkTask* t, const WideUnit* u, int n
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int g = n < 2 * sms ? n : 2 * sms;   // persistent: two CTAs per SM walk the units
+    const int g = n < sms ? n : sms;   // persistent: one CTA per SM (146 KB of stages) walks the units
     if (mode == 0)
     {
         cudaError_t e = allow_smem(k_blk_wide<0>, b);
