@@ -497,10 +497,22 @@ int build_plan(h2gpu_image* im, const h2gpu_desc* d, HostPlan& hp)
     // into tasks of a multiple of 64 rows).  A task's kernel walks its rows in chunks
     // of 64 and adds the chunks' transposed products into the task's single slot, so
     // a block has one A^T w slot per task instead of one per 64-row chunk.
-    const int RB = 1024;
-    auto rows_per_task = [&](int nr) {
+    // Images with fewer blocks than CTA slots (148 SMs x 3) take smaller tasks, down to
+    // one chunk, so that the launch covers the GPU (Coulomb N = 1,501: 36 blocks, their launch 19 -> 10 us).
+    auto rows_per_task = [](int nr, int RB) {
         const int nt = (nr + RB - 1) / RB;
         return ((nr + nt - 1) / nt + 63) / 64 * 64;
+    };
+    auto task_rows = [&](int n, const int* nrow, const int* ncol) {
+        int RB = 1024;
+        for (; RB > 64; RB /= 2)
+        {
+            long long tasks = 0;
+            for (int i = 0; i < n && tasks < 444; i++)
+                if (nrow[i] > 0 && ncol[i] > 0) tasks += (nrow[i] + rows_per_task(nrow[i], RB) - 1) / rows_per_task(nrow[i], RB);
+            if (tasks >= 444) break;
+        }
+        return RB;
     };
     std::vector<BlkTask>& blkB = hp.blkB;
     std::vector<BlkTask>& blkD = hp.blkD;
@@ -519,6 +531,7 @@ int build_plan(h2gpu_image* im, const h2gpu_desc* d, HostPlan& hp)
             im->bmap[0].push_back({(long long) d->B_ptr[i], off32B[i], d->B_nrow[i], d->B_ncol[i]});
         for (int i = 0; i < d->n_D; i++)
             im->bmap[1].push_back({(long long) d->D_ptr[i], off32D[i], d->D_nrow[i], d->D_ncol[i]});
+        const int RB_B = task_rows(d->n_B, d->B_nrow, d->B_ncol), RB_D = task_rows(d->n_D, d->D_nrow, d->D_ncol);
         for (int i = 0; i < d->n_B; i++)
         {
             int n0 = d->r_adm_pairs[2 * i], n1 = d->r_adm_pairs[2 * i + 1];
@@ -534,7 +547,7 @@ int build_plan(h2gpu_image* im, const h2gpu_desc* d, HostPlan& hp)
             int in1 = (l0 < l1) ? mc[2 * n0] : N + y0r[n0];
             int s0 = alloc(nr);
             if (l0 < l1) asms[n0].push_back(s0); else { y1s[n0].push_back(s0); }
-            const int R = rows_per_task(nr);
+            const int R = rows_per_task(nr, RB_B);
             for (int r0 = 0; r0 < nr; r0 += R)
             {
                 int rr = std::min(R, nr - r0);
@@ -558,7 +571,7 @@ int build_plan(h2gpu_image* im, const h2gpu_desc* d, HostPlan& hp)
             bool diag = i < d->n_leaf_node;
             int s0 = alloc(nr);
             asms[n0].push_back(s0);
-            const int R = rows_per_task(nr);
+            const int R = rows_per_task(nr, RB_D);
             for (int r0 = 0; r0 < nr; r0 += R)
             {
                 int rr = std::min(R, nr - r0);
@@ -589,8 +602,11 @@ int build_plan(h2gpu_image* im, const h2gpu_desc* d, HostPlan& hp)
                 n64 += cls(t) == 0;
                 n32 += cls(t) <= 1;
             }
-            im->blk1_small[li][0] = n64;
-            im->blk1_small[li][1] = n32;
+            // a warp per task needs more tasks than the GPU has warp slots to pay: with fewer
+            // than two per CTA slot every task is a CTA's
+            const bool few = ts.size() < 2 * 444;
+            im->blk1_small[li][0] = few ? 0 : n64;
+            im->blk1_small[li][1] = few ? 0 : n32;
         }
         // units of the 64-wide passes: pass 0 per 128-row chunk of a task (A V), pass 1 per
         // 128-column tile of a task (A^T W)
