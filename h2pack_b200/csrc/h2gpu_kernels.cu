@@ -822,35 +822,45 @@ __global__ void __launch_bounds__(kThreads) k_down(const DownTask* __restrict__ 
     }
 }
 
-// Sum of one element over n slots, in slot order, eight loads in flight.
-__device__ __forceinline__ double slot_sum(const double* __restrict__ p, const int* __restrict__ sl, int n, int NV)
+// Sum of one element (V = double) or of two neighbours (double2) over n slots, in slot
+// order, eight loads in flight; stride: the slots' rows in units of V.
+__device__ __forceinline__ void add_to(double& s, double a) { s += a; }
+__device__ __forceinline__ void add_to(double2& s, double2 a) { s.x += a.x; s.y += a.y; }
+template <typename V>
+__device__ __forceinline__ V slot_sum(const V* __restrict__ p, const int* __restrict__ sl, int n, int stride)
 {
-    double s = 0.0;
+    V s{};
     int k = 0;
     for (; k + 8 <= n; k += 8)
     {
-        double a[8];
+        V a[8];
 #pragma unroll
-        for (int u = 0; u < 8; u++) a[u] = p[(long long) sl[k + u] * NV];
+        for (int u = 0; u < 8; u++) a[u] = p[(long long) sl[k + u] * stride];
 #pragma unroll
-        for (int u = 0; u < 8; u++) s += a[u];
+        for (int u = 0; u < 8; u++) add_to(s, a[u]);
     }
-    for (; k < n; k++) s += p[(long long) sl[k] * NV];
+    for (; k < n; k++) add_to(s, p[(long long) sl[k] * stride]);
     return s;
 }
 
 // The slot sums are bound by HBM (each slot row is read once); what kept them from it was
 // one CTA per node walking its elements one after the other, each a chain of dependent
 // load / add steps.  The elements of a node are spread over gridDim.y CTAs
-// (sum_grid_y) and slot_sum keeps eight loads in flight.
+// (sum_grid_y) and slot_sum keeps eight loads in flight (of two right-hand sides each, but
+// for a single one).  RPY N = 20,011, 64 right-hand sides: k_asm 5.20 -> 0.41 ms, k_y1sum 1.13
+// -> 0.42; Matern N = 1M, 16: k_asm 0.114 -> 0.075 with pairs.
 // y1 of a node = sum of its PS slots (fixed order); rows indexed like the y0 region.
 template <int NV>
 __global__ void k_y1sum(const Y1Task* __restrict__ tasks, const int* __restrict__ slots,
                         const double* __restrict__ PS, double* __restrict__ Y1)
 {
+    using V = typename std::conditional<NV == 1, double, double2>::type;
+    constexpr int ST = NV == 1 ? 1 : NV / 2;
     const Y1Task t = tasks[blockIdx.x];
-    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < t.nrow * NV; i += blockDim.x * gridDim.y)
-        Y1[(long long) t.row * NV + i] = slot_sum(PS + i, slots + t.slot_beg, t.slot_end - t.slot_beg, NV);
+    const V* const ps = reinterpret_cast<const V*>(PS);
+    V* const y = reinterpret_cast<V*>(Y1) + (long long) t.row * ST;
+    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < t.nrow * ST; i += blockDim.x * gridDim.y)
+        y[i] = slot_sum(ps + i, slots + t.slot_beg, t.slot_end - t.slot_beg, ST);
 }
 
 // --------------------------------------------------------------- assemble
@@ -861,13 +871,22 @@ __global__ void k_asm(const AsmTask* __restrict__ tasks, const int* __restrict__
                       const double* __restrict__ PS, const int* __restrict__ fwd,
                       double* __restrict__ Y, long long y_rs, long long y_cs, int nv)
 {
+    using V = typename std::conditional<NV == 1, double, double2>::type;
+    constexpr int ST = NV == 1 ? 1 : NV / 2;
     const AsmTask t = tasks[blockIdx.x];
-    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < t.nrow * NV; i += blockDim.x * gridDim.y)
+    const V* const ps = reinterpret_cast<const V*>(PS);
+    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < t.nrow * ST; i += blockDim.x * gridDim.y)
     {
-        int r = i / NV, v = i % NV;
+        const int r = i / ST, v = NV == 1 ? 0 : 2 * (i % ST);
         if (v >= nv) continue;
-        Y[(long long) fwd[t.row0 + r] * y_rs + (long long) v * y_cs] =
-            slot_sum(PS + i, slots + t.slot_beg, t.slot_end - t.slot_beg, NV);
+        const V s = slot_sum(ps + i, slots + t.slot_beg, t.slot_end - t.slot_beg, ST);
+        double* const y = Y + (long long) fwd[t.row0 + r] * y_rs + (long long) v * y_cs;
+        if constexpr (NV == 1) *y = s;
+        else
+        {
+            *y = s.x;
+            if (v + 1 < nv) y[y_cs] = s.y;
+        }
     }
 }
 
@@ -4209,11 +4228,11 @@ cudaError_t launch_down(int NV, const DownTask* t, int n, const TA* U, const dou
     return cudaGetLastError();
 }
 
-// CTAs per task of the slot sums: one element per thread for an average task, as long as
+// CTAs per task of the slot sums: one element (pair) per thread for an average task, as long as
 // that stays within 32 CTAs per SM in all (beyond it the launch is HBM-bound anyway).
 static int sum_grid_y(int n, long long rows, int NV)
 {
-    const long long per = (rows * NV / n + 255) / 256, most = (148 * 32 + n - 1) / n;
+    const long long per = (rows * ((NV + 1) / 2) / n + 255) / 256, most = (148 * 32 + n - 1) / n;
     return (int) (per < 1 ? 1 : per < most ? per : most);
 }
 

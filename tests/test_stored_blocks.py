@@ -1,0 +1,38 @@
+"""Stored blocks (k_blk1, the 64-wide passes, the panels between) against the same product in
+64-bit torch from the same representation (perf/cases.py): images with fewer blocks than CTA
+slots (tasks of 64-row chunks) and with more, blocks of odd sizes below and above one tile
+of 64 and one unit of 128, level-mismatched pairs, every panel width and remainder.
+
+Tolerance: FP64 as the on-the-fly path's (1e-13); mixed 2e-6 (FP32 blocks, BF16x3 or 3xTF32
+products with FP32 sums of at most 64 terms).
+"""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("kernel,n,leaf", [("coulomb", 20, 100), ("coulomb", 1501, 300), ("coulomb", 2003, 40),
+                                           ("gaussian", 5000, 700), ("matern32", 12007, 150), ("rpy", 130, 50),
+                                           ("rpy", 3001, 60)])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_matches_64_bit_product(kernel, n, leaf, precision):
+    import torch
+    from perf import cases
+    case = {"kind": "apply", "kernel": kernel, "n": n, "leaf": leaf, "mode": "generate", "precision": precision, "api": "device"}
+    rep = cases.Rep(case, n, 4)
+    img = cases.Image(rep.describe(), precision, blocks="generate")
+    X = cases._rhs(case, rep.kd * n, 128, 4)
+    Y = rep.apply(X)
+    tol = 1e-13 if precision == "fp64" else 2e-6
+    for nv in (1, 2, 3, 4, 8, 16, 20, 33, 64, 100):
+        y = img.matmul_device(X[:, :nv].contiguous())
+        torch.cuda.synchronize()
+        assert float((y - Y[:, :nv]).norm() / Y[:, :nv].norm()) < tol, nv
+    # host calls: through the pinned buffer and past its size, both layouts
+    import numpy as np
+    Xh, Yh = X.cpu().numpy(), Y.cpu().numpy()
+    assert np.linalg.norm(img.matvec(Xh[:, 0]) - Yh[:, 0]) < tol * np.linalg.norm(Yh[:, 0])
+    for layout in (101, 102):
+        for nv in (2, 17):
+            assert np.linalg.norm(img.matmul(Xh[:, :nv], layout) - Yh[:, :nv]) < tol * np.linalg.norm(Yh[:, :nv])
+    img.close()
