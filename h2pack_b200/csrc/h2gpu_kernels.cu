@@ -915,6 +915,12 @@ __device__ __forceinline__ float rsqrt_approx(float x)
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+__device__ __forceinline__ float sqrt_approx(float x)
+{
+    float y;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
 constexpr float kLog2e = 1.4426950408889634f;
 
 template <> struct Math<float> {
@@ -931,6 +937,9 @@ template <typename T> struct Scalar<KRNL_COULOMB_ID, T> {
 template <typename T> struct Scalar<KRNL_GAUSSIAN_ID, T> {
     static __device__ __forceinline__ T f(T r2, T p0, T) { return Math<T>::exp_(-p0 * r2); }
 };
+template <> struct Scalar<KRNL_GAUSSIAN_ID, float> {
+    static __device__ __forceinline__ float f(float r2, float p0, float) { return ex2_approx(r2 * (-p0 * kLog2e)); }
+};
 template <typename T> struct Scalar<KRNL_MATERN32_ID, T> {
     static __device__ __forceinline__ T f(T r2, T, T c0)
     {
@@ -938,11 +947,13 @@ template <typename T> struct Scalar<KRNL_MATERN32_ID, T> {
         return (T(1) - t) * Math<T>::exp_(t);
     }
 };
-// (1 - t) e^t = e - t e with e = 2^(t log2 e): 7 instructions, 2 of them MUFU
+// (1 - t) e^t = e - t e with e = 2^(t log2 e): 5 instructions, 2 of them MUFU (the hardware
+// square root, also right at r = 0, in place of r^2 rsqrt(r^2) behind a maximum: near and far field of
+// Matern N = 1M, 16 right-hand sides, 38.0 -> 36.9 ms, error 4.7e-7 as before)
 template <> struct Scalar<KRNL_MATERN32_ID, float> {
     static __device__ __forceinline__ float f(float r2, float, float c0)
     {
-        float t = c0 * (r2 * rsqrt_approx(fmaxf(r2, 1e-30f)));
+        float t = c0 * sqrt_approx(r2);
         float e = ex2_approx(t * kLog2e);
         return fmaf(-t, e, e);
     }
@@ -960,16 +971,16 @@ template <> struct ScalarF2<KRNL_COULOMB_ID> {
 template <> struct ScalarF2<KRNL_GAUSSIAN_ID> {
     static __device__ __forceinline__ float2 f2(float2 r2, float p0, float)
     {
-        // exp(-p0 r^2) = 2^((-p0 r^2) log2 e)
-        const float2 t = __fmul2_rn(__fmul2_rn(make_float2(-p0, -p0), r2), make_float2(kLog2e, kLog2e));
+        // exp(-p0 r^2) = 2^(r^2 (-p0 log2 e))
+        const float q = -p0 * kLog2e;
+        const float2 t = __fmul2_rn(r2, make_float2(q, q));
         return make_float2(ex2_approx(t.x), ex2_approx(t.y));
     }
 };
 template <> struct ScalarF2<KRNL_MATERN32_ID> {
     static __device__ __forceinline__ float2 f2(float2 r2, float, float c0)
     {
-        const float2 rs = make_float2(rsqrt_approx(fmaxf(r2.x, 1e-30f)), rsqrt_approx(fmaxf(r2.y, 1e-30f)));
-        const float2 t = __fmul2_rn(make_float2(c0, c0), __fmul2_rn(r2, rs));
+        const float2 t = __fmul2_rn(make_float2(c0, c0), make_float2(sqrt_approx(r2.x), sqrt_approx(r2.y)));
         const float2 u = __fmul2_rn(t, make_float2(kLog2e, kLog2e));
         const float2 e = make_float2(ex2_approx(u.x), ex2_approx(u.y));
         return __ffma2_rn(make_float2(-t.x, -t.y), e, e);
@@ -1016,7 +1027,7 @@ template <> struct ScalarFar<KRNL_MATERN32_ID> {
     static __device__ __forceinline__ void prep(float, float, float& q0, float& q1) { q0 = 0.6931471805599453f; q1 = 0.f; }
     static __device__ __forceinline__ float2 f2(float2 r2s, float ln2, float)
     {
-        const float2 s = __fmul2_rn(r2s, make_float2(rsqrt_approx(r2s.x), rsqrt_approx(r2s.y)));
+        const float2 s = make_float2(sqrt_approx(r2s.x), sqrt_approx(r2s.y));
         const float2 e = make_float2(ex2_approx(-s.x), ex2_approx(-s.y));
         return __fmul2_rn(__ffma2_rn(s, make_float2(ln2, ln2), make_float2(1.f, 1.f)), e);
     }
