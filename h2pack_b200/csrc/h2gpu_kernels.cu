@@ -1066,6 +1066,16 @@ template <typename T> struct Vec4;
 template <> struct Vec4<double> { using t = double4; };
 template <> struct Vec4<float> { using t = float4; };
 
+// Part `part` of `parts` of a target chunk (of <= 128 targets); npt <= 0 past its end.
+__device__ __forceinline__ JitTarget chunk_part(JitTarget t, int part, int parts, int kd)
+{
+    const int w = 128 / parts;
+    t.pt0 += part * w;
+    t.out_row += kd * part * w;
+    t.npt = min(w, t.npt - part * w);
+    return t;
+}
+
 // The CTAs of a cluster that share a target chunk (jit_split) add their sums in the first
 // one: n values of this thread, at v + k * stride of its CTA's shared memory, the other
 // CTAs' values at the same place of theirs (distributed shared memory), in rank order.
@@ -1347,7 +1357,7 @@ template <int NV, int KD> struct Jit64Cfg {
 template <int KID, int NV, int KD>
 __global__ void __launch_bounds__(Jit64Cfg<NV, KD>::NT, Jit64Cfg<NV, KD>::CTAS)
     k_jit64(const JitTarget* __restrict__ tgts, const TileRec* __restrict__ tiles, const double4* __restrict__ pts,
-            KParam kp, const double* __restrict__ XS, double* __restrict__ PS, double* __restrict__ Y1, int S)
+            KParam kp, const double* __restrict__ XS, double* __restrict__ PS, double* __restrict__ Y1, int parts, int S)
 {
     namespace cg = cooperative_groups;
     using C = Jit64Cfg<NV, KD>;
@@ -1355,8 +1365,9 @@ __global__ void __launch_bounds__(Jit64Cfg<NV, KD>::NT, Jit64Cfg<NV, KD>::CTAS)
     __shared__ __align__(16) double s_tab[16];
     __shared__ __align__(16) double4 s_pt[TILE];
     __shared__ __align__(16) double s_buf[C::BUF];
-    const int rank = (int) (blockIdx.x & (S - 1));
-    const JitTarget tg = tgts[blockIdx.x / S];
+    const int rank = (int) (blockIdx.x & (S - 1)), unit = blockIdx.x / S;
+    const JitTarget tg = chunk_part(tgts[unit / parts], unit % parts, parts, KD);
+    if (tg.npt <= 0) return;                   // the whole cluster
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, q = lane & 3, row = lane >> 2;
     // warps with targets, shares of the sources, this warp's targets and how many groups of 8
     const int nw = (tg.npt + WT - 1) / WT, ns = NWARP / nw;
@@ -4265,17 +4276,28 @@ cudaError_t launch_asm(int NV, const AsmTask* t, int n, const int* slots, const 
     return cudaGetLastError();
 }
 
-// CTAs per target chunk (the CTAs of a cluster share a chunk's source tiles): the smallest
-// power of two that gives the launch two waves of the SMs' CTA slots, at most 8 (the portable
-// cluster size).  Two waves: with one, near fields of 1,063 chunks (FP64, N = 120,000) took
-// 2.23 instead of 2.05 ms and the served case below 38.1 instead of 37.4; with four, a far
-// field of 1,216 chunks 10.9 instead of 9.6 ms.  FP32: 16 requests on a Gaussian matrix of N =
-// 20,011 (192 near chunks on 592 slots): 60.8 -> 37.4 ms.
-static int jit_split(int n, int per_sm)
+// How a launch of n target chunks covers the SMs' CTA slots.  parts: CTAs that each take
+// 128 / parts of a chunk's targets (against all its sources; the warps left over share the
+// sources), until the launch has four waves; share: the CTAs of a cluster that share the
+// sources of one such part, up to 8 (the portable cluster size), until it has two.
+// FP64: halves at most.  Matern N = 120,000, 16 right-hand sides (far field of 1,216 chunks, 2.05
+// waves): 11.84 -> 11.06 ms, quarters 11.18; N = 100,000, 1: 6.02 -> 5.71; RPY N = 20,011, 1: 0.90
+// -> 0.86; Gaussian N = 10,007: 0.23 with quarters 0.25.
+// FP32: whole chunks (the tensor-core kernel's FP64 flush per 64 sources is paid by every
+// warp that shares them: Matern N = 125,000, 16: 3.7 ms, halves 4.6).
+// share, two waves: with one, near fields of 1,063 chunks (FP64, N = 120,000) took 2.23
+// instead of 2.05 ms and the served case below 38.1 instead of 37.4; with four, a far field of
+// 1,216 chunks 10.9 instead of 9.6 ms; by a model of waves and tiles, with any number up to 8,
+// Matern N = 120,000 13.4 instead of 11.9.  FP32: 16 requests on a Gaussian matrix of N = 20,011
+// (192 near chunks on 592 slots): 60.8 -> 37.4 ms.
+struct JitSplit { int parts, share; };
+static JitSplit jit_split(int n, int per_sm, int max_parts)
 {
-    int S = 1;
-    while (S < 8 && (long long) n * S < 2LL * 148 * per_sm) S *= 2;
-    return S;
+    const long long slots = 148LL * per_sm;
+    JitSplit s{1, 1};
+    while (s.parts < max_parts && n * s.parts < 4 * slots) s.parts *= 2;
+    while (s.share < 8 && (long long) n * s.parts * s.share < 2 * slots) s.share *= 2;
+    return s;
 }
 
 // n * S CTAs in clusters of S
@@ -4325,7 +4347,7 @@ static cudaError_t launch_jit_k(int NV, const JitTarget* tg, int n, const void* 
                                  : (far ? k_jit_tc<KID, 8, true> : k_jit_tc<KID, 8, false>);
             cudaError_t e = allow_smem(kern, b);
             if (e != cudaSuccess) return e;
-            const int S = jit_split(n, 4);
+            const int S = jit_split(n, 4, 1).share;
             return launch_cluster(kern, n, S, 256, b, st, tg, tiles, p4, ppts, pin, kp, PS, Y1, lo, plo, S);
         }
     }
@@ -4337,21 +4359,22 @@ static cudaError_t launch_jit_k(int NV, const JitTarget* tg, int n, const void* 
             return cudaErrorInvalidValue;   // tensor kernels run in panels of <= 8 right-hand sides
         else if constexpr (sizeof(T) == 8)
         {
-            const int S = jit_split(n, 4);
-            return launch_cluster(k_jit64<KID, NVc, KD>, n, S, Jit64Cfg<NVc, KD>::NT, 0, st, tg, tiles, p, kp, XS, PS, Y1, S);
+            const JitSplit sp = jit_split(n, 4, 2);
+            return launch_cluster(k_jit64<KID, NVc, KD>, n * sp.parts, sp.share, Jit64Cfg<NVc, KD>::NT, 0, st, tg, tiles, p,
+                                  kp, XS, PS, Y1, sp.parts, sp.share);
         }
         else if constexpr (KD == 1 && sizeof(T) == 4)
         {
             // scalar FP32 kernels: the two targets of a thread as one FP32x2 pair
             if (!use_shift) return cudaErrorInvalidValue;   // FP32 evaluation is re-centred
-            const int S = jit_split(n, 8);
+            const int S = jit_split(n, 8, 1).share;
             return launch_cluster(far ? k_jit2<KID, NVc, true> : k_jit2<KID, NVc, false>, n, S, 64, 0, st, tg, tiles,
                                   (const float4*) pts, kp, XS, PS, Y1, lo, S);
         }
         else
         {
             constexpr int TPT = KD * NVc <= 16 ? 2 : 1;
-            const int S = jit_split(n, 5 * TPT);
+            const int S = jit_split(n, 5 * TPT, 1).share;
             return launch_cluster(k_jit<KID, NVc, KD, TPT>, n, S, 128 / TPT, 0, st, tg, tiles, p, kp, use_shift, XS, PS, Y1, S);
         }
     });
