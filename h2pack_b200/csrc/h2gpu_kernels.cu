@@ -391,10 +391,11 @@ __device__ __forceinline__ void chunk_apply(const TA* __restrict__ A, int R, int
 //
 // A warp walks its rows eight at a time.  What bounds it is how many bytes a warp keeps on
 // their way.
-// FP64 (H2Pack's packing, rows on 8 bytes): the lane owns columns lane + 32 j, a pass of 32
+// FP64 (H2Pack's packing, rows on 8 bytes): the lane owns columns lane + 32 j, two passes of 32
 // columns at a time; their A^T w sums live in the warp's row of shared memory (only the lane
-// touches its columns: no barrier).  24 warps per SM; requesting the next pass during a pass
-// took registers from the warps and measured slower (B phase 0.61 -> 0.69 ms at N = 80,000).
+// touches its columns: no barrier).  24 warps per SM (Coulomb N = 80,000: B phase 0.61 -> 0.59 ms
+// against one pass at a time; requesting the next pass during a pass 0.69, two passes in 16
+// warps per SM 0.60 and the near field a fifth slower).
 // FP32 (rows padded to 16 bytes): the lane owns four columns of each 128, 16 bytes a load,
 // both passes' sums and inputs in registers; a group's entries are requested while the group
 // before it is multiplied and reduced.  Coulomb N = 80,000, mixed: B phase 0.43 -> 0.33 ms, the
@@ -420,22 +421,31 @@ __device__ __forceinline__ void blk1_warp(const BlkTask& T, const double* __rest
 #pragma unroll
         for (int k = 0; k < 8; k++) p[k] = 0.0;
 #pragma unroll 1
-        for (int j = 0; j < J; j++)
+        for (int j = 0; j < J; j += 2)
         {
-            const int c = lane + 32 * j;
-            const bool cv = c < ncol;
-            double a[8];
+            const int c = lane + 32 * j, c2 = c + 32;
+            const bool cv = c < ncol, cv2 = c2 < ncol;
+            double a[8], b[8];
 #pragma unroll
-            for (int k = 0; k < 8; k++) a[k] = (cv && k < nr) ? A[(long long) (r0 + k) * ncol + c] : 0.0;
-            const double v = (do0 && cv) ? XS[T.in0_row + c] : 0.0;
-            double q = 0.0;
+            for (int k = 0; k < 8; k++) a[k] = (cv && k < nr) ? __ldg(A + (long long) (r0 + k) * ncol + c) : 0.0;
+#pragma unroll
+            for (int k = 0; k < 8; k++) b[k] = (cv2 && k < nr) ? __ldg(A + (long long) (r0 + k) * ncol + c2) : 0.0;
+            const double v = (do0 && cv) ? XS[T.in0_row + c] : 0.0, v2 = (do0 && cv2) ? XS[T.in0_row + c2] : 0.0;
+            double q = 0.0, q2 = 0.0;
 #pragma unroll
             for (int k = 0; k < 8; k++)
             {
                 q = fma(a[k], wr[k], q);
                 p[k] = fma(a[k], v, p[k]);
             }
+#pragma unroll
+            for (int k = 0; k < 8; k++)
+            {
+                q2 = fma(b[k], wr[k], q2);
+                p[k] = fma(b[k], v2, p[k]);
+            }
             sq[c] += q;
+            if (cv2) sq[c2] += q2;
         }
         if (do0)
         {
