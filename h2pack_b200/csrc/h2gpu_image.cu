@@ -114,6 +114,14 @@ struct h2gpu_image {
     BlkTask* d_blkB = nullptr;
     BlkTask* d_blkD = nullptr;
     WideUnit* d_wide = nullptr;   // units of the 64-wide passes: B pass 0, B pass 1, D pass 0, D pass 1
+    WideSeg* d_wseg = nullptr;
+    // their slot sums, and the partial rows that the 64-wide panels use
+    Y1Task* d_y1tw = nullptr;
+    int* d_y1_slotsw = nullptr;
+    AsmTask* d_asmw = nullptr;
+    int* d_asm_slotsw = nullptr;
+    int n_y1w = 0, n_asmw = 0;
+    long long ps_wide = 0;
     int n_wide[4] = {0, 0, 0, 0};
     JitTarget* d_jtN = nullptr;
     JitTarget* d_jtF = nullptr;
@@ -206,7 +214,8 @@ void free_all(h2gpu_image* im)
                     im->d_B32, im->d_D64, im->d_D32, im->d_pts64, im->d_pts32, im->d_XS, im->d_PS, im->d_Y1,
                     im->d_PUSH, im->d_io, im->d_owN, im->d_owF, im->d_pp, im->d_jtN2, im->d_jtF2, im->d_y1t2,
                     im->d_y1_slots2, im->d_asm2, im->d_asm_slots2, im->d_status, im->d_pg, im->d_ppts,
-                    im->d_pin, im->d_tiles, im->d_wide, im->d_XS3, im->d_pts32lo, im->d_pplo};
+                    im->d_pin, im->d_tiles, im->d_wide, im->d_wseg, im->d_y1tw, im->d_y1_slotsw, im->d_asmw,
+                    im->d_asm_slotsw, im->d_XS3, im->d_pts32lo, im->d_pplo};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (im->h_status) cudaFreeHost(im->h_status);
@@ -367,6 +376,11 @@ struct HostPlan {
     std::vector<int> y1_slots;
     std::vector<BlkTask> blkB, blkD;
     std::vector<WideUnit> wide;   // B pass 0, B pass 1, D pass 0, D pass 1 (counts in n_wide)
+    std::vector<WideSeg> wseg;
+    std::vector<Y1Task> y1tw;
+    std::vector<int> y1_slotsw;
+    std::vector<AsmTask> atw;
+    std::vector<int> at_slotsw;
     std::vector<JitTarget> jtN, jtF;
     std::vector<JitSource> js;
     std::vector<AsmTask> at;
@@ -488,13 +502,33 @@ int build_plan(h2gpu_image* im, const h2gpu_desc* d, HostPlan& hp)
     im->up_beg.push_back((int) up.size());
     im->n_up = (int) up.size();
 
-    // ---- partial slots
+    // ---- partial slots: the leaves' downward results first (every plan of the image uses
+    // them), then each plan's own
     long long ps = 0;
     auto alloc = [&](int rows) { long long r = ps; ps += rows; return (int) r; };
+    std::vector<int> leaf_dst(n_node, -1);
+    {
+        // a node has a downward result when it or a node above it has y1 contributions
+        std::vector<char> down(n_node, 0);
+        for (int i = 0; i < d->n_r_adm_pair; i++)
+        {
+            const int a = d->r_adm_pairs[2 * i], b = d->r_adm_pairs[2 * i + 1];
+            if (lvl[a] >= lvl[b]) down[a] = 1;
+            if (lvl[b] >= lvl[a]) down[b] = 1;
+        }
+        for (int L = min_adm; L <= d->max_level; L++)
+            for (int j = 0; j < d->level_n_node[L]; j++)
+            {
+                const int n = d->level_nodes[(size_t) L * d->n_leaf_node + j];
+                if (parent[n] >= 0 && lvl[parent[n]] >= min_adm && down[parent[n]]) down[n] = 1;
+                if (down[n] && d->n_child[n] == 0 && d->U_nrow[n] > 0 && d->U_ncol[n] > 0) leaf_dst[n] = alloc(d->U_nrow[n]);
+            }
+    }
+    long long psw = ps;   // slots of the 64-wide plan, which shares the rows after these
     std::vector<std::vector<int>> y1s(n_node), asms(n_node);
     // pair plan slots of a node: (slot, first row) -- a slot of the node's full size
     // (first row -1), or one of an owner unit covering rows [first row, + 128) of it
-    std::vector<std::vector<std::pair<int, int>>> pair_y1, pair_asm;
+    std::vector<std::vector<std::pair<int, int>>> pair_y1, pair_asm, wide_y1, wide_asm;
     std::vector<char> has_y1(n_node, 0);
     // Stored blocks: one task per block of up to RB rows (larger blocks split evenly
     // into tasks of a multiple of 64 rows).  A task's kernel walks its rows in chunks
@@ -611,31 +645,82 @@ int build_plan(h2gpu_image* im, const h2gpu_desc* d, HostPlan& hp)
             im->blk1_small[li][0] = few ? 0 : n64;
             im->blk1_small[li][1] = few ? 0 : n32;
         }
-        // units of the 64-wide passes: pass 0 per 128-row chunk of a task (A V), pass 1 per
-        // 128-column tile of a task (A^T W)
-        // Pass-0 units are ordered by their input rows (the column node's y0 / x slice),
-        // so that consecutive units, walked by the persistent CTAs in order, read the same
-        // 64-wide input rows from L2; pass-1 units read their task's own rows and keep the
-        // task order (tasks of one row node are adjacent).
-        auto units = [&](const std::vector<BlkTask>& ts, int pass) {
-            std::vector<WideUnit> us;
-            for (int i = 0; i < (int) ts.size(); i++)
+        // units of the 64-wide passes (WideUnit).  An owner is a node's y1 rows or a leaf's
+        // output rows; its blocks are cut into runs of at most a share of all tiles (about
+        // four units per SM), so that the persistent CTAs end together.
+        wide_y1.assign(n_node, {});
+        wide_asm.assign(n_node, {});
+        auto units = [&](bool isB, int pass) {
+            const int nb = isB ? d->n_B : d->n_D;
+            const std::vector<long long>& off = isB ? off32B : off32D;
+            std::vector<std::vector<int>> own_y1(n_node), own_asm(n_node);
+            long long total = 0;
+            auto nodes_of = [&](int i, int& n0, int& n1) {
+                if (isB) { n0 = d->r_adm_pairs[2 * i]; n1 = d->r_adm_pairs[2 * i + 1]; }
+                else if (i < d->n_leaf_node) n0 = n1 = d->leaf_nodes[i];
+                else
+                {
+                    n0 = d->r_inadm_pairs[2 * (i - d->n_leaf_node)];
+                    n1 = d->r_inadm_pairs[2 * (i - d->n_leaf_node) + 1];
+                }
+            };
+            auto nr_of = [&](int i) { return isB ? d->B_nrow[i] : d->D_nrow[i]; };
+            auto nc_of = [&](int i) { return isB ? d->B_ncol[i] : d->D_ncol[i]; };
+            for (int i = 0; i < nb; i++)
             {
-                const BlkTask& t = ts[i];
-                if ((pass == 0 ? t.out0_row : t.out1_row) < 0) continue;
-                for (int o = 0; o < (pass == 0 ? t.nrow : t.ncol); o += kWideRows) us.push_back(WideUnit{i, o});
+                if (nr_of(i) == 0 || nc_of(i) == 0 || (!isB && i < d->n_leaf_node && pass == 1)) continue;
+                int n0, n1;
+                nodes_of(i, n0, n1);
+                const bool y1 = isB && (pass == 0 ? lvl[n0] >= lvl[n1] : lvl[n1] >= lvl[n0]);
+                (y1 ? own_y1 : own_asm)[pass == 0 ? n0 : n1].push_back(i);
+                const int M = pass == 0 ? nr_of(i) : nc_of(i), K = pass == 0 ? nc_of(i) : nr_of(i);
+                total += (long long) ((M + kWideRows - 1) / kWideRows) * ((K + 63) / 64);
             }
-            if (pass == 0)
-                std::stable_sort(us.begin(), us.end(), [&](const WideUnit& a, const WideUnit& b) {
-                    return ts[a.task].in0_row < ts[b.task].in0_row;
-                });
+            const long long cap = std::max<long long>(16, total / (148 * 4));
+            std::vector<WideUnit> us;
+            for (int kind = 0; kind < 2; kind++)
+                for (int n = 0; n < n_node; n++)
+                {
+                    const std::vector<int>& list = (kind == 0 ? own_y1 : own_asm)[n];
+                    if (list.empty()) continue;
+                    const int R = pass == 0 ? nr_of(list[0]) : nc_of(list[0]);
+                    for (int c0 = 0; c0 < R; c0 += kWideRows)
+                        for (size_t k = 0; k < list.size();)
+                        {
+                            WideUnit u;
+                            u.seg_beg = (int) hp.wseg.size();
+                            u.rows = std::min(kWideRows, R - c0);
+                            u.out_row = (int) psw;
+                            psw += u.rows;
+                            u.nt = 0;
+                            do {
+                                const int i = list[k++];
+                                int n0, n1;
+                                nodes_of(i, n0, n1);
+                                const int src = pass == 0 ? n1 : n0, oth = pass == 0 ? n0 : n1;
+                                WideSeg g;
+                                g.ld = f32_ld(nc_of(i));
+                                g.a = off[i] + (pass == 0 ? (long long) c0 * g.ld : c0);
+                                g.K = pass == 0 ? nc_of(i) : nr_of(i);
+                                // a coarser source gives its points' input, otherwise its skeleton's
+                                g.in_row = !isB || lvl[src] < lvl[oth] ? mc[2 * src] : N + y0r[src];
+                                g.pad = 0;
+                                hp.wseg.push_back(g);
+                                u.nt += (g.K + 63) / 64;
+                            } while (k < list.size() && u.nt < cap);
+                            u.seg_end = (int) hp.wseg.size();
+                            us.push_back(u);
+                            (kind == 0 ? wide_y1 : wide_asm)[n].push_back({u.out_row, c0});
+                        }
+                }
+            std::stable_sort(us.begin(), us.end(), [](const WideUnit& x, const WideUnit& y) { return x.nt > y.nt; });
             hp.wide.insert(hp.wide.end(), us.begin(), us.end());
             return (int) us.size();
         };
-        im->n_wide[0] = units(blkB, 0);
-        im->n_wide[1] = units(blkB, 1);
-        im->n_wide[2] = units(blkD, 0);
-        im->n_wide[3] = units(blkD, 1);
+        im->n_wide[0] = units(true, 0);
+        im->n_wide[1] = units(true, 1);
+        im->n_wide[2] = units(false, 0);
+        im->n_wide[3] = units(false, 1);
     } else {
         // ---- JIT: point space = sorted points, then the skeleton points of every node
         std::vector<double> half;
@@ -1013,9 +1098,10 @@ int build_plan(h2gpu_image* im, const h2gpu_desc* d, HostPlan& hp)
             if (!has_y1[n] && !push) continue;
             done[n] = 1;
             bool leaf = d->n_child[n] == 0;
-            int dst = leaf ? alloc(nr) : y0r[d->children[n * d->max_child]];
+            int dst = leaf ? leaf_dst[n] : y0r[d->children[n * d->max_child]];
             if (leaf) asms[n].push_back(dst);
             if (leaf && !pair_asm.empty()) pair_asm[n].push_back({dst, -1});
+            if (leaf && !wide_asm.empty()) wide_asm[n].push_back({dst, -1});
             const int RD = 64;       // downward tasks: one 64-row chunk of U each
             for (int r0 = 0; r0 < nr; r0 += RD)
             {
@@ -1046,7 +1132,7 @@ int build_plan(h2gpu_image* im, const h2gpu_desc* d, HostPlan& hp)
         t.slot_end = (int) at_slots.size();
         at.push_back(t);
     }
-    if (im->has_pair)
+    if (im->has_pair || !wide_asm.empty())
     {
         // one sum per 128-row piece of a node: the owner units' slots of that piece and
         // the same piece of every full-size slot, in the order the slots were made
@@ -1060,26 +1146,33 @@ int build_plan(h2gpu_image* im, const h2gpu_desc* d, HostPlan& hp)
                 add(c0, std::min(kPairOwnerChunk, rows - c0), beg, (int) slots.size());
             }
         };
+        static_assert(kPairOwnerChunk == kWideRows, "pieces");
+        const auto& ey1 = im->has_pair ? pair_y1 : wide_y1;
+        const auto& easm = im->has_pair ? pair_asm : wide_asm;
+        auto& sy1 = im->has_pair ? hp.y1_slots2 : hp.y1_slotsw;
+        auto& sasm = im->has_pair ? hp.at_slots2 : hp.at_slotsw;
         for (int n = 0; n < n_node; n++)
         {
             if (!has_y1[n]) continue;
-            pieces(pair_y1[n], d->U_ncol[n], hp.y1_slots2, [&](int c0, int len, int b, int e) {
-                hp.y1t2.push_back(Y1Task{y0r[n] + c0, len, b, e});
+            pieces(ey1[n], d->U_ncol[n], sy1, [&](int c0, int len, int b, int e) {
+                (im->has_pair ? hp.y1t2 : hp.y1tw).push_back(Y1Task{y0r[n] + c0, len, b, e});
             });
         }
         for (int i = 0; i < d->n_leaf_node; i++)
         {
             int n = d->leaf_nodes[i];
-            pieces(pair_asm[n], kd * npt_of(d, n), hp.at_slots2, [&](int c0, int len, int b, int e) {
-                hp.at2.push_back(AsmTask{mc[2 * n] + c0, len, b, e});
+            pieces(easm[n], kd * npt_of(d, n), sasm, [&](int c0, int len, int b, int e) {
+                (im->has_pair ? hp.at2 : hp.atw).push_back(AsmTask{mc[2 * n] + c0, len, b, e});
             });
         }
+        im->n_y1w = (int) hp.y1tw.size(); im->n_asmw = (int) hp.atw.size();
         im->n_asm2 = (int) hp.at2.size();
         im->n_owN = (int) hp.owN.size(); im->n_owF = (int) hp.owF.size();
         im->n_jtN2 = (int) hp.jtN2.size(); im->n_jtF2 = (int) hp.jtF2.size(); im->n_y12 = (int) hp.y1t2.size();
     }
-    REQ(ps < (1LL << 31), "partial space too large");
-    im->ps_rows = ps;
+    REQ(ps < (1LL << 31) && psw < (1LL << 31), "partial space too large");
+    im->ps_rows = std::max(ps, psw);
+    im->ps_wide = psw;
 
     // ---- statistics of the algorithm (per right-hand side)
     double ub = 0, bb = 0, db = 0, fwd = 0, mid = 0, bwd = 0, den = 0, pB = 0, pD = 0;
@@ -1374,32 +1467,51 @@ int check_plan(const h2gpu_image* im, const h2gpu_desc* d, const HostPlan& hp, l
         TRY(cover_blocks("B", hp.blkB, d->n_B, d->B_nrow, d->B_ncol, d->B_ptr));
         TRY(cover_blocks("D", hp.blkD, d->n_D, d->D_nrow, d->D_ncol, d->D_ptr));
         // ---- units of the 64-wide passes: every 128-row chunk (pass 0) and every 128-column
-        //      tile (pass 1) of every task that has the product, once each
+        //      chunk (pass 1; not of diagonal blocks) of every block once, inside its arena;
+        //      the units' slots written and summed once
         long long w0 = 0;
         const int* nw = im->n_wide;
         REQ((long long) hp.wide.size() == (long long) nw[0] + nw[1] + nw[2] + nw[3], "plan: wide unit counts");
+        std::vector<std::pair<long long, long long>> prodw = down_ps;
         for (int part = 0; part < 4; part++)
         {
-            const std::vector<BlkTask>& ts = part < 2 ? hp.blkB : hp.blkD;
+            const std::vector<h2gpu_image::BlkMap>& bm = im->bmap[part < 2 ? 0 : 1];
             const int pass = part & 1;
-            std::vector<std::vector<char>> seen(ts.size());
+            std::vector<std::vector<char>> seen(bm.size());
             for (long long k = w0; k < w0 + nw[part]; k++)
             {
                 const WideUnit u = hp.wide[k];
-                REQ(u.task >= 0 && u.task < (int) ts.size(), "plan: a wide unit names no task");
-                const BlkTask& t = ts[u.task];
-                const int ext = pass == 0 ? t.nrow : t.ncol;
-                REQ((pass == 0 ? t.out0_row : t.out1_row) >= 0, "plan: a wide unit of a product its task lacks");
-                REQ(u.off >= 0 && u.off < ext && u.off % kWideRows == 0, "plan: a wide unit starts off its grid");
-                if (seen[u.task].empty()) seen[u.task].assign((ext + kWideRows - 1) / kWideRows, 0);
-                REQ(++seen[u.task][u.off / kWideRows] == 1, "plan: a wide unit repeats");
+                REQ(u.rows >= 1 && u.rows <= kWideRows, "plan: a wide unit of %d rows", u.rows);
+                REQ(u.seg_beg >= 0 && u.seg_beg < u.seg_end && u.seg_end <= (int) hp.wseg.size(), "plan: a wide unit without segments");
+                prodw.push_back({u.out_row, u.rows});
+                REQ((long long) u.out_row + u.rows <= im->ps_wide, "plan: a wide slot outside its partial space");
+                int nt = 0;
+                for (int g = u.seg_beg; g < u.seg_end; g++)
+                {
+                    const WideSeg& sg = hp.wseg[g];
+                    auto it = std::upper_bound(bm.begin(), bm.end(), sg.a, [](long long v, const h2gpu_image::BlkMap& m) { return v < m.off32; });
+                    // empty blocks share their offset with the next one
+                    REQ(it != bm.begin(), "plan: a wide segment before its arena");
+                    const size_t i = (size_t) (it - bm.begin()) - 1;
+                    const int M = pass == 0 ? bm[i].nrow : bm[i].ncol, K = pass == 0 ? bm[i].ncol : bm[i].nrow, ld = f32_ld(bm[i].ncol);
+                    const long long o = sg.a - bm[i].off32, r0 = pass == 0 ? o / ld : o;
+                    REQ(sg.ld == ld && sg.K == K && (pass == 1 || o % ld == 0) && r0 % kWideRows == 0 && r0 < M &&
+                            u.rows == std::min(kWideRows, (int) (M - r0)),
+                        "plan: a wide segment does not match its block");
+                    REQ(sg.in_row >= 0 && (long long) sg.in_row + K <= N + Y0, "plan: wide input outside the input space");
+                    if (seen[i].empty()) seen[i].assign((M + kWideRows - 1) / kWideRows, 0);
+                    REQ(++seen[i][r0 / kWideRows] == 1, "plan: a wide segment repeats");
+                    nt += (K + 63) / 64;
+                }
+                REQ(nt == u.nt, "plan: a wide unit's tile count");
             }
-            for (size_t i = 0; i < ts.size(); i++)
-                if ((pass == 0 ? ts[i].out0_row : ts[i].out1_row) >= 0)
+            for (size_t i = 0; i < bm.size(); i++)
+                if (bm[i].nrow > 0 && bm[i].ncol > 0 && !(part == 3 && i < (size_t) d->n_leaf_node))
                     REQ(!seen[i].empty() && std::count(seen[i].begin(), seen[i].end(), 1) == (long long) seen[i].size(),
-                        "plan: a task's %s is not covered by wide units", pass == 0 ? "rows" : "columns");
+                        "plan: a block's %s are not covered by wide units", pass == 0 ? "rows" : "columns");
             w0 += nw[part];
         }
+        TRY(check_space("64-wide", prodw, {}, hp.atw, hp.at_slotsw, hp.y1tw, hp.y1_slotsw));
     }
 
     long long pairs_plan = 0;
@@ -1652,6 +1764,11 @@ int upload_plan(h2gpu_image* im, const h2gpu_desc* d, HostPlan& hp)
     TRY(upload(hp.blkB, &im->d_blkB, im->bytes));
     TRY(upload(hp.blkD, &im->d_blkD, im->bytes));
     TRY(upload(hp.wide, &im->d_wide, im->bytes));
+    TRY(upload(hp.wseg, &im->d_wseg, im->bytes));
+    TRY(upload(hp.y1tw, &im->d_y1tw, im->bytes));
+    TRY(upload(hp.y1_slotsw, &im->d_y1_slotsw, im->bytes));
+    TRY(upload(hp.atw, &im->d_asmw, im->bytes));
+    TRY(upload(hp.at_slotsw, &im->d_asm_slotsw, im->bytes));
     TRY(upload(hp.jtN, &im->d_jtN, im->bytes));
     TRY(upload(hp.jtF, &im->d_jtF, im->bytes));
     TRY(upload(hp.at, &im->d_asm, im->bytes));
@@ -1752,7 +1869,9 @@ int ensure_work(h2gpu_image* im, int NV)
     if (im->d_XS3) { cudaFree(im->d_XS3); im->d_XS3 = nullptr; }
     im->NVb = 0;          // no buffers until all four are allocated
     im->work_bytes = 0;
-    size_t xs = ((size_t) im->N + im->y0_rows) * NV, ps = (size_t) im->ps_rows * NV, y1 = (size_t) im->y0_rows * NV;
+    // 64-wide panels use the rows of their own plan; narrower ones, of up to 32, all
+    const size_t ps = NV == 64 ? std::max((size_t) im->ps_wide * 64, (size_t) im->ps_rows * 32) : (size_t) im->ps_rows * NV;
+    size_t xs = ((size_t) im->N + im->y0_rows) * NV, y1 = (size_t) im->y0_rows * NV;
     CK(cudaMalloc(&im->d_XS, 8 * std::max<size_t>(xs, 1)));
     CK(cudaMalloc(&im->d_PS, 8 * std::max<size_t>(ps, 1)));
     CK(cudaMalloc(&im->d_Y1, 8 * std::max<size_t>(y1, 1)));
@@ -1919,17 +2038,18 @@ int run_panel(h2gpu_image* im, int NV, int nv, const double* X, long long x_rs, 
         {
             const int* nw = im->n_wide;
             CK(launch_split3(im->d_XS, im->N, im->y0_rows, xs_rows, im->d_XS3, c));   // the skeleton rows y0
-            CK(launch_blk_wide(0, im->d_blkB, im->d_wide, nw[0], im->d_B32, im->d_XS3, xs_rows, im->d_PS, c,
+            CK(launch_blk_wide(0, im->d_wide, nw[0], im->d_wseg, im->d_B32, im->d_XS3, xs_rows, im->d_PS, c,
                                im->d_status));
-            CK(launch_blk_wide(1, im->d_blkB, im->d_wide + nw[0], nw[1], im->d_B32, im->d_XS3, xs_rows, im->d_PS, c,
+            CK(launch_blk_wide(1, im->d_wide + nw[0], nw[1], im->d_wseg, im->d_B32, im->d_XS3, xs_rows, im->d_PS, c,
                                im->d_status));
+            CK(launch_y1sum(NV, im->d_y1tw, im->n_y1w, im->d_y1_slotsw, im->d_PS, im->d_Y1, im->y0_rows, c));
             im->st.n_launches += 2;   // the second pass and the split of the inputs
         }
         else if (f32) CK(launch_blk<float>(NV, im->d_blkB, im->n_blkB, im->d_B32, im->d_XS, im->d_PS, c, im->blk_tc, im->d_status,
                                            im->blk1_small[0][1]));
         else CK(launch_blk<double>(NV, im->d_blkB, im->n_blkB, im->d_B64, im->d_XS, im->d_PS, c, 0, nullptr,
                                    im->blk1_small[0][0]));
-        CK(launch_y1sum(NV, im->d_y1t, im->n_y1, im->d_y1_slots, im->d_PS, im->d_Y1, im->y0_rows, c));
+        if (!wide) CK(launch_y1sum(NV, im->d_y1t, im->n_y1, im->d_y1_slots, im->d_PS, im->d_Y1, im->y0_rows, c));
     } else {
         if (panels) CK(launch_panel_in(NV, im->d_pg, im->n_pg_pts, im->n_pg - im->n_pg_pts, im->d_XS, im->d_pin, c));
         CK(launch_jit(im->kernel_id, f32, NV, im->d_jtF, im->n_jtF, f32 ? (const void*) im->d_pts32 : (const void*) im->d_pts64,
@@ -1951,9 +2071,9 @@ int run_panel(h2gpu_image* im, int NV, int nv, const double* X, long long x_rs, 
         if (wide)
         {
             const int* nw = im->n_wide;
-            CK(launch_blk_wide(0, im->d_blkD, im->d_wide + nw[0] + nw[1], nw[2], im->d_D32, im->d_XS3, xs_rows,
+            CK(launch_blk_wide(0, im->d_wide + nw[0] + nw[1], nw[2], im->d_wseg, im->d_D32, im->d_XS3, xs_rows,
                                im->d_PS, s, im->d_status));
-            CK(launch_blk_wide(1, im->d_blkD, im->d_wide + nw[0] + nw[1] + nw[2], nw[3], im->d_D32, im->d_XS3,
+            CK(launch_blk_wide(1, im->d_wide + nw[0] + nw[1] + nw[2], nw[3], im->d_wseg, im->d_D32, im->d_XS3,
                                xs_rows, im->d_PS, s, im->d_status));
             im->st.n_launches += 2;   // the second pass and the split of the inputs
         }
@@ -1969,8 +2089,8 @@ int run_panel(h2gpu_image* im, int NV, int nv, const double* X, long long x_rs, 
     }
     if (timed) CK(cudaEventRecord(e[2], s));
     CK(cudaStreamWaitEvent(s, im->ev_join, 0));
-    CK(launch_asm(NV, im->d_asm, im->n_asm, im->d_asm_slots, im->d_PS, im->d_fwd, Y, y_rs, y_cs, nv, im->N,
-                  s));
+    if (wide) CK(launch_asm(NV, im->d_asmw, im->n_asmw, im->d_asm_slotsw, im->d_PS, im->d_fwd, Y, y_rs, y_cs, nv, im->N, s));
+    else CK(launch_asm(NV, im->d_asm, im->n_asm, im->d_asm_slots, im->d_PS, im->d_fwd, Y, y_rs, y_cs, nv, im->N, s));
     if (timed && uses_status(im, NV))
         CK(cudaMemcpyAsync(im->h_status, im->d_status, sizeof(int), cudaMemcpyDeviceToHost, s));
     if (timed) CK(cudaEventRecord(e[6], s));

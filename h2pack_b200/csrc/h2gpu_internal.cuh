@@ -80,13 +80,22 @@ __host__ __device__ inline bool blk1_fits(int nrow, int ncol, int elem_bytes)
     return ncol <= kBlk1WarpCols && nrow <= kBlk1WarpRows && (long long) nrow * ncol * elem_bytes <= kBlk1WarpBytes;
 }
 
-// Unit of the wide-panel stored-block passes: one 128-row chunk of a task (pass 0,
-// A V over all column tiles) or one 128-column tile of a task (pass 1, A^T W over all of
-// the task's rows).
+// Wide-panel stored-block passes (64 right-hand sides).  A unit is <= 128 output rows of a
+// node and a run of the blocks that add to them, so that its sums stay in registers over all
+// of them: pass 0 (A V) the blocks in whose row node the rows lie, pass 1 (A^T W) those in
+// whose column node.  A segment is one block's part: its first entry (row, or column, of the
+// unit's first output row) in the FP32 arena, its row stride, the summed dimension and its
+// input rows.  A node's slots are the units' (WideUnit::out_row), few per 128 rows, instead of
+// one per block.
 constexpr int kWideRows = 128;
 struct WideUnit {
-    int task;          // index into the block-task list
-    int off;           // first row (pass 0) or first column (pass 1) of the unit
+    int seg_beg, seg_end;
+    int nt;            // tiles of 64 of the summed dimension, over all segments
+    int rows, out_row; // output rows, PS row of the first
+};
+struct WideSeg {
+    long long a;
+    int ld, K, in_row, pad;
 };
 
 // JIT target: a set of points whose outputs accumulate over a list of source sets

@@ -3075,11 +3075,10 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16_ab(int n, int a_mn_major,
            ((uint32_t) (n >> 3) << 17) | ((uint32_t) (128 >> 4) << 24);
 }
 
-// A panel of 64 right-hand sides applied to the stored blocks as two passes over the block
-// tasks, each a plain GEMM whose outputs are written once (the one-pass kernel's per-tile
-// read-modify-write of the transposed-product slot dominated its memory traffic):
-//   pass 0, one unit per 128-row chunk of a task:     C0 = A_chunk V    (over the column tiles)
-//   pass 1, one unit per 128-column tile of a task:   C1 = A_tile^T W   (over the task's rows)
+// A panel of 64 right-hand sides applied to the stored blocks as two passes, each a plain
+// GEMM whose outputs stay in registers over all blocks that add to them (WideUnit):
+//   pass 0, <= 128 rows of a node:     C += A_rows V       over the blocks of that row node
+//   pass 1, <= 128 rows of a node:     C += (A_cols)^T W   over the blocks of that column node
 // A unit is walked in tiles of 64 along the summed dimension.  Each 128 x 64 (64 x 128) tile
 // of A (FP32) is split into BF16 pieces h + m + l in shared memory (128-byte rows, 128-byte
 // swizzle).  The right-hand sides of a tile (64 rows of the input space, row-major with the
@@ -3087,13 +3086,15 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16_ab(int n, int a_mn_major,
 // they are copied as they are.  Six products per 16-deep K step (l.h + h.l + m.m + m.h + h.m
 // + h.h), FP32 in TMEM over one tile (64 terms), FP64 across tiles in registers.
 //
-// What bounds it: blocks of 100 to 400 rows and columns are one to four tiles per unit, so
-// any step that waits for the step before it is exposed once or twice a unit (64-row units
-// with all threads taking the steps in turn: 5.7 us per 16 KB tile).  The roles are separate
+// What bounds it: a tile's steps (load, split, 24 MMAs, FP64 sums) depend on each other, so
+// any that waits in turn is exposed every tile (all threads taking the steps in turn: 5.7 us
+// per 16 KB tile).  The roles are separate
 // warps that run ahead of each other through two stages, across units: 8 warps load A
 // (one tile ahead, in registers) and split it, one thread issues the MMAs, 8 warps read the
 // products and sum.  RPY N = 20,011, 64 right-hand sides: the two passes over B 6.0 -> 3.7 ms,
-// the matmul 8.3 -> 5.05.  Bounded waits record a status and stop.
+// the matmul 8.3 -> 5.05.  Units over all blocks of a node instead of one block
+// (no slot per block to write and sum): 5.05 -> 3.31 ms.
+// Bounded waits record a status and stop.
 struct WideSmem {
     uint16_t a[2][3][128 * 64];   // two stages of A tile pieces
     uint16_t b[2][3][64 * 64];    // two stages of right-hand-side pieces: 64 rows (k) of 64 BF16
@@ -3151,54 +3152,57 @@ __global__ void k_split3(const double* __restrict__ XS, long long row0, long lon
     }
 }
 
-// One unit of a pass, and its walk by a persistent CTA: units blockIdx.x, + gridDim.x, ..
-template <int MODE>
+// A persistent CTA's walk over the units blockIdx.x, + gridDim.x, .. of a pass, tile by tile
+// of their segments; the next segment's record is read a segment ahead.
 struct WideWalk {
-    const BlkTask* tasks;
     const WideUnit* units;
-    int n, ui;          // units; the current one
-    BlkTask T, Tn;      // its task; the next unit's, read one unit ahead
-    int off, offn, nt;  // first row (column) of the unit; its tiles
-    __device__ __forceinline__ void read_next()
+    const WideSeg* segs;
+    int n, ui, si, t;
+    WideUnit U, Un;     // the current unit, the next one
+    WideSeg S, Sn;      // the current segment, the next one (of the next unit after the last)
+    __device__ __forceinline__ void ahead()
     {
-        if (ui + (int) gridDim.x < n)
-        {
-            const WideUnit U = units[ui + gridDim.x];
-            Tn = tasks[U.task];
-            offn = U.off;
-        }
+        if (si + 1 < U.seg_end) Sn = segs[si + 1];
+        else if (ui + (int) gridDim.x < n) Sn = segs[Un.seg_beg];
     }
-    __device__ __forceinline__ void take()
+    __device__ __forceinline__ void next_unit()
     {
-        T = Tn;
-        off = offn;
-        nt = ((MODE == 0 ? T.ncol : T.nrow) + 63) / 64;
-        read_next();
+        if (ui + (int) gridDim.x < n) Un = units[ui + gridDim.x];
     }
-    __device__ __forceinline__ bool begin(const BlkTask* t, const WideUnit* u, int count)
+    __device__ __forceinline__ bool begin(const WideUnit* u, int count, const WideSeg* sg)
     {
-        tasks = t; units = u; n = count;
-        ui = (int) blockIdx.x - (int) gridDim.x;
-        if ((int) blockIdx.x >= n) return false;
-        read_next();
-        ui += gridDim.x;
-        take();
+        units = u; segs = sg; n = count;
+        ui = blockIdx.x;
+        if (ui >= n) return false;
+        U = units[ui];
+        next_unit();
+        si = U.seg_beg;
+        S = segs[si];
+        t = 0;
+        ahead();
         return true;
     }
     __device__ __forceinline__ bool next()
     {
-        ui += gridDim.x;
-        if (ui >= n) return false;
-        take();
+        if (64 * ++t < S.K) return true;
+        t = 0;
+        S = Sn;
+        if (++si == U.seg_end)
+        {
+            ui += gridDim.x;
+            if (ui >= n) return false;
+            U = Un;
+            si = U.seg_beg;
+            next_unit();
+        }
+        ahead();
         return true;
     }
-    // rows (pass 0) or columns (pass 1) of the unit
-    __device__ __forceinline__ int extent() const { return min(128, (MODE == 0 ? T.nrow : T.ncol) - off); }
 };
 
 template <int MODE>
-__global__ void __launch_bounds__(kWideThreads, 1) k_blk_wide(const BlkTask* __restrict__ tasks,
-                                                              const WideUnit* __restrict__ units, int n_units,
+__global__ void __launch_bounds__(kWideThreads, 1) k_blk_wide(const WideUnit* __restrict__ units, int n_units,
+                                                              const WideSeg* __restrict__ segs,
                                                               const float* __restrict__ arena,
                                                               const uint16_t* __restrict__ XS3, long long rows3,
                                                               double* __restrict__ PS, int* __restrict__ status)
@@ -3247,16 +3251,16 @@ __global__ void __launch_bounds__(kWideThreads, 1) k_blk_wide(const BlkTask* __r
     auto arrive = [&](unsigned long long* bar) {
         asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.shared::cta.b64 t, [%0];\n\t}" ::"r"(smem_u32(bar)) : "memory");
     };
-    WideWalk<MODE> w;
     if (warp < 8)
     {
         // ---- loaders.  A: four granules of 8 consecutive values of a row per thread, as two
         // 16-byte loads each (FP32 rows are padded to 16 bytes with zeros, so a vector that
         // starts before the row's end stays in the row); zeros outside the unit.
+        WideWalk w;
         float4 ra[4][2];
-        auto load_a = [&](int t) {
-            const int M = w.extent(), K = min(64, (MODE == 0 ? w.T.ncol : w.T.nrow) - 64 * t), ld = w.T.ld32;
-            const float* A = arena + w.T.a32 + (MODE == 0 ? (long long) w.off * ld + 64 * t : (long long) (64 * t) * ld + w.off);
+        auto load_a = [&]() {
+            const int M = w.U.rows, K = min(64, w.S.K - 64 * w.t), ld = w.S.ld;
+            const float* A = arena + w.S.a + (MODE == 0 ? (long long) (64 * w.t) : (long long) (64 * w.t) * ld);
 #pragma unroll
             for (int u = 0; u < 4; u++)
             {
@@ -3286,14 +3290,14 @@ __global__ void __launch_bounds__(kWideThreads, 1) k_blk_wide(const BlkTask* __r
                 *reinterpret_cast<uint4*>(a_b + 2 * PIECE_A + off) = make_uint4(l[0], l[1], l[2], l[3]);
             }
         };
-        bool more = w.begin(tasks, units, n_units);
-        if (more) load_a(0);
-        for (int i = 0, t = 0; more; i++)
+        bool more = w.begin(units, n_units, segs);
+        if (more) load_a();
+        for (int i = 0; more; i++)
         {
             const int st = i & 1;
             if (i >= 2 && !wait(&sm.empty[st], ((i >> 1) - 1) & 1)) break;
-            const int nk = min(64, (MODE == 0 ? w.T.ncol : w.T.nrow) - 64 * t);
-            const long long row0 = (long long) (MODE == 0 ? w.T.in0_row : w.T.in1_row) + 64 * t;
+            const int nk = min(64, w.S.K - 64 * w.t);
+            const long long row0 = (long long) w.S.in_row + 64 * w.t;
 #pragma unroll
             for (int u = 0; u < 6; u++)
             {
@@ -3303,12 +3307,8 @@ __global__ void __launch_bounds__(kWideThreads, 1) k_blk_wide(const BlkTask* __r
             }
             cp_async_commit();
             store_a(st);
-            if (++t == w.nt)
-            {
-                t = 0;
-                more = w.next();
-            }
-            if (more) load_a(t);                 // in flight until the next tile's split
+            more = w.next();
+            if (more) load_a();                  // in flight until the next tile's split
             cp_async_wait_all();
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             arrive(&sm.full[st]);
@@ -3321,10 +3321,11 @@ __global__ void __launch_bounds__(kWideThreads, 1) k_blk_wide(const BlkTask* __r
         const int quad = warp & 3, half = (warp - 8) >> 2;
         double acc[32];
         int i = 0;
-        for (bool more = w.begin(tasks, units, n_units); more; more = w.next())
+        for (int ui = blockIdx.x; ui < n_units; ui += gridDim.x)
         {
+            const WideUnit U = units[ui];
             bool ok = true;
-            for (int t = 0; t < w.nt; t++, i++)
+            for (int t = 0; t < U.nt; t++, i++)
             {
                 const int d = i & 1;
                 if (!(ok = __all_sync(kFull, wait(&sm.tfull[d], (i >> 1) & 1)))) break;   // the loads below are the warp's
@@ -3351,10 +3352,10 @@ __global__ void __launch_bounds__(kWideThreads, 1) k_blk_wide(const BlkTask* __r
             }
             if (!ok) break;
             const int m = 32 * quad + lane;
-            if (m < w.extent())
+            if (m < U.rows)
             {
                 // 16 bytes a store: rows of 64 doubles, 32 of them this thread's
-                double2* o = reinterpret_cast<double2*>(PS + (long long) ((MODE == 0 ? w.T.out0_row : w.T.out1_row) + w.off + m) * NV + 32 * half);
+                double2* o = reinterpret_cast<double2*>(PS + (long long) (U.out_row + m) * NV + 32 * half);
 #pragma unroll
                 for (int n = 0; n < 16; n++) o[n] = make_double2(acc[2 * n], acc[2 * n + 1]);
             }
@@ -3366,8 +3367,8 @@ __global__ void __launch_bounds__(kWideThreads, 1) k_blk_wide(const BlkTask* __r
         constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};
         int i = 0;
         bool ok = true;
-        for (bool more = w.begin(tasks, units, n_units); more && ok; more = w.next())
-            for (int t = 0; t < w.nt; t++, i++)
+        for (int ui = blockIdx.x; ui < n_units && ok; ui += gridDim.x)
+            for (int t = 0, nt = units[ui].nt; t < nt; t++, i++)
             {
                 const int st = i & 1;
                 if (!(ok = wait(&sm.full[st], (i >> 1) & 1))) break;
@@ -4207,7 +4208,7 @@ cudaError_t launch_split3(const double* XS, long long row0, long long n, long lo
     return cudaGetLastError();
 }
 
-cudaError_t launch_blk_wide(int mode, const BlkTask* t, const WideUnit* u, int n, const float* arena,
+cudaError_t launch_blk_wide(int mode, const WideUnit* u, int n, const WideSeg* segs, const float* arena,
                             const uint16_t* XS3, long long rows3, double* PS, cudaStream_t st, int* status)
 {
     if (n <= 0) return cudaSuccess;
@@ -4221,11 +4222,11 @@ cudaError_t launch_blk_wide(int mode, const BlkTask* t, const WideUnit* u, int n
     {
         cudaError_t e = allow_smem(k_blk_wide<0>, b);
         if (e != cudaSuccess) return e;
-        k_blk_wide<0><<<g, kWideThreads, b, st>>>(t, u, n, arena, XS3, rows3, PS, status);
+        k_blk_wide<0><<<g, kWideThreads, b, st>>>(u, n, segs, arena, XS3, rows3, PS, status);
     } else {
         cudaError_t e = allow_smem(k_blk_wide<1>, b);
         if (e != cudaSuccess) return e;
-        k_blk_wide<1><<<g, kWideThreads, b, st>>>(t, u, n, arena, XS3, rows3, PS, status);
+        k_blk_wide<1><<<g, kWideThreads, b, st>>>(u, n, segs, arena, XS3, rows3, PS, status);
     }
     return cudaGetLastError();
 }

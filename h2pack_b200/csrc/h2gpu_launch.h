@@ -19,9 +19,9 @@ template <typename TA>
 cudaError_t launch_blk(int NV, const BlkTask* t, int n, const TA* arena, const double* XS, double* PS, cudaStream_t st,
                        int use_tc = 0, int* status = nullptr,    // use_tc: 1 mma.sync, 2 tcgen05
                        int n_small = 0);   // NV 1: leading tasks that blk1_fits for TA (one warp each)
-// 64-wide panels of FP32 stored blocks on tcgen05: pass 0 (mode 0, units = 128-row chunks:
-// A V) or pass 1 (mode 1, units = 128-column tiles: A^T W), outputs written once
-cudaError_t launch_blk_wide(int mode, const BlkTask* t, const WideUnit* u, int n, const float* arena,
+// 64-wide panels of FP32 stored blocks on tcgen05: pass 0 (mode 0, A V) or pass 1 (mode 1,
+// A^T W), units of 128 output rows over all their blocks
+cudaError_t launch_blk_wide(int mode, const WideUnit* u, int n, const WideSeg* segs, const float* arena,
                             const uint16_t* XS3, long long rows3, double* PS, cudaStream_t st, int* status);
 // rows [row0, row0 + n) of the 64-wide input space (row stride 64) into its BF16 pieces
 cudaError_t launch_split3(const double* XS, long long row0, long long n, long long rows, uint16_t* XS3,
