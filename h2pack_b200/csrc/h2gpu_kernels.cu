@@ -1086,22 +1086,28 @@ __device__ __forceinline__ JitTarget chunk_part(JitTarget t, int part, int parts
     return t;
 }
 
-// The CTAs of a cluster that share a target chunk (jit_split) add their sums in the first
-// one: n values of this thread, at v + k * stride of its CTA's shared memory, the other
-// CTAs' values at the same place of theirs (distributed shared memory), in rank order.
+// The CTAs of a cluster that share a target chunk (jit_split) add their sums: of the n values
+// of this thread, at v + k * stride of its CTA's shared memory and at the same place of the
+// other CTAs', CTA `rank` adds and keeps those with k = rank (mod S), in rank order (distributed
+// shared memory; all of them in the first CTA was a chain of 7 remote reads per value: 16
+// requests on a Gaussian matrix of N = 20,011 32.3 -> 28.6 ms).
 // Called by every thread of the cluster; the memory may be reused after it returns.
 __device__ __forceinline__ void cluster_sum(double* v, int stride, int n, int rank, int S)
 {
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
     cl.sync();
-    if (rank == 0)
-        for (int r = 1; r < S; r++)
-        {
-            const double* o = cl.map_shared_rank(v, r);
-#pragma unroll 4
-            for (int k = 0; k < n; k++) v[k * stride] += o[k * stride];
-        }
+    for (int k = rank; k < n; k += S)
+    {
+        double a[8];
+#pragma unroll
+        for (int r = 0; r < 8; r++) a[r] = r < S ? cl.map_shared_rank(v, r)[k * stride] : 0.0;
+        double s = a[0];
+#pragma unroll
+        for (int r = 1; r < 8; r++)
+            if (r < S) s += a[r];
+        v[k * stride] = s;
+    }
     cl.sync();
 }
 
@@ -1210,7 +1216,6 @@ __global__ void __launch_bounds__(128 / TPT, 5 * TPT) k_jit(const JitTarget* __r
         }
     }
     if (S > 1) cluster_sum(s_acc + threadIdx.x, NT, TPT * W, rank, S);
-    if (rank != 0) return;
 #pragma unroll
     for (int q = 0; q < TPT; q++)
     {
@@ -1219,7 +1224,7 @@ __global__ void __launch_bounds__(128 / TPT, 5 * TPT) k_jit(const JitTarget* __r
         double* o = (tg.out_y1 ? Y1 : PS) + (long long) (tg.out_row + KD * i) * NV;
 #pragma unroll
         for (int k = 0; k < W; k++)
-            o[k] = s_acc[(q * W + k) * NT + threadIdx.x];
+            if (((q * W + k) & (S - 1)) == rank) o[k] = s_acc[(q * W + k) * NT + threadIdx.x];
     }
 }
 
@@ -1557,19 +1562,16 @@ __global__ void __launch_bounds__(Jit64Cfg<NV, KD>::NT, Jit64Cfg<NV, KD>::CTAS)
         }
     __syncthreads();
     if (S > 1) cg::this_cluster().sync();
-    if (rank == 0)
+    double* const out = (tg.out_y1 ? Y1 : PS) + (long long) tg.out_row * NV;
+    for (int e = tid + NT * rank; e < tg.npt * W; e += NT * S)
     {
-        double* const out = (tg.out_y1 ? Y1 : PS) + (long long) tg.out_row * NV;
-        for (int e = tid; e < tg.npt * W; e += NT)
+        double s = 0.0;
+        for (int r = 0; r < S; r++)
         {
-            double s = 0.0;
-            for (int r = 0; r < S; r++)
-            {
-                const double* b = S > 1 ? cg::this_cluster().map_shared_rank(s_buf, r) : s_buf;
-                for (int g = 0; g < ns; g++) s += b[g * nw * WT * W + e];
-            }
-            out[e] = s;
+            const double* b = S > 1 ? cg::this_cluster().map_shared_rank(s_buf, r) : s_buf;
+            for (int g = 0; g < ns; g++) s += b[g * nw * WT * W + e];
         }
+        out[e] = s;
     }
     if (S > 1) cg::this_cluster().sync();      // shared memory stays until it has been read
 }
@@ -1694,13 +1696,12 @@ __global__ void __launch_bounds__(64, NV >= 16 ? 8 : 10) k_jit2(const JitTarget*
         }
     }
     if (S > 1) cluster_sum(&s_acc[0][threadIdx.x], NT, 2 * NV, rank, S);
-    if (rank != 0) return;
     double* o = tg.out_y1 ? Y1 : PS;
 #pragma unroll
     for (int v = 0; v < NV; v++)
     {
-        if (v0) o[(long long) (tg.out_row + i0) * NV + v] = s_acc[v][threadIdx.x];
-        if (v1) o[(long long) (tg.out_row + i1) * NV + v] = s_acc[NV + v][threadIdx.x];
+        if (v0 && (v & (S - 1)) == rank) o[(long long) (tg.out_row + i0) * NV + v] = s_acc[v][threadIdx.x];
+        if (v1 && ((NV + v) & (S - 1)) == rank) o[(long long) (tg.out_row + i1) * NV + v] = s_acc[NV + v][threadIdx.x];
     }
 }
 
@@ -2007,7 +2008,6 @@ __global__ void __launch_bounds__(256, 4) k_jit_tc(const JitTarget* __restrict__
     }
     // the sums of the chunk's other CTAs, in rank order
     if (S > 1) cluster_sum(&sm.acc[warp][0][lane], 32, 8, rank, S);
-    if (rank != 0) return;
     // accumulator (n, q) of lane (g, t): right-hand side g + 8 (q >> 1), target
     // 16w + 8n + 2t + (q & 1)
     double* base = (tg.out_y1 ? Y1 : PS) + (long long) tg.out_row * NV;
@@ -2017,7 +2017,8 @@ __global__ void __launch_bounds__(256, 4) k_jit_tc(const JitTarget* __restrict__
         for (int q = 0; q < 4; q++)
         {
             const int row = warp * 16 + 8 * n + 2 * tq + (q & 1), rhs = g + 8 * (q >> 1);
-            if (row < tg.npt && rhs < NV) base[(long long) row * NV + rhs] = sm.acc[warp][n * 4 + q][lane];
+            if (row < tg.npt && rhs < NV && ((n * 4 + q) & (S - 1)) == rank)
+                base[(long long) row * NV + rhs] = sm.acc[warp][n * 4 + q][lane];
         }
 }
 
@@ -4297,7 +4298,7 @@ cudaError_t launch_asm(int NV, const AsmTask* t, int n, const int* slots, const 
 // FP32: whole chunks (the tensor-core kernel's FP64 flush per 64 sources is paid by every
 // warp that shares them: Matern N = 125,000, 16: 3.7 ms, halves 4.6).
 // share, two waves: with one, near fields of 1,063 chunks (FP64, N = 120,000) took 2.23
-// instead of 2.05 ms and the served case below 38.1 instead of 37.4; with four, a far field of
+// instead of 2.05 ms and the served case below 38.1 instead of 37.4 (before cluster_sum); with four, a far field of
 // 1,216 chunks 10.9 instead of 9.6 ms; by a model of waves and tiles, with any number up to 8,
 // Matern N = 120,000 13.4 instead of 11.9.  FP32: 16 requests on a Gaussian matrix of N = 20,011
 // (192 near chunks on 592 slots): 60.8 -> 37.4 ms.
