@@ -1952,6 +1952,9 @@ bool pair_plan(const h2gpu_image* im, int NV)
     return im->has_pair && im->jit_pair && im->precision == H2GPU_PREC_MIXED && im->jit_tc && (NV == 8 || NV == 16);
 }
 
+// Whether an apply has sweeps or a far field at all (not when no pair of nodes is admissible).
+bool has_chain(const h2gpu_image* im) { return im->n_up > 0 || im->n_dn > 0 || im->n_blkB > 0 || im->n_jtF > 0; }
+
 // One panel of NV right-hand sides: X (original order, strides x_rs, x_cs) -> Y.
 int run_panel(h2gpu_image* im, int NV, int nv, const double* X, long long x_rs, long long x_cs, double* Y,
               long long y_rs, long long y_cs, cudaStream_t s, bool timed)
@@ -2016,55 +2019,58 @@ int run_panel(h2gpu_image* im, int NV, int nv, const double* X, long long x_rs, 
     CK(launch_gather(NV, X, x_rs, x_cs, nv, im->d_fwd, im->N, im->d_XS, s));
     if (wide) CK(launch_split3(im->d_XS, 0, im->N, xs_rows, im->d_XS3, s));
     if (panels) CK(launch_panel_in(NV, im->d_pg, 0, im->n_pg_pts, im->d_XS, im->d_pin, s));
-    CK(cudaEventRecord(im->ev_fork, s));
     if (timed) CK(cudaEventRecord(e[1], s));
-    CK(cudaStreamWaitEvent(c, im->ev_fork, 0));
-    for (size_t L = 0; L + 1 < im->up_beg.size(); L++)
+    if (has_chain(im))
     {
-        int b = im->up_beg[L], n = im->up_beg[L + 1] - b;
-        if (f32) CK(launch_up<float>(NV, im->d_up + b, n, im->d_U32, im->d_XS, c, sweep_tc(im)));
-        else CK(launch_up<double>(NV, im->d_up + b, n, im->d_U64, im->d_XS, c));
-    }
-    if (timed) CK(cudaEventRecord(e[3], c));
-    if (im->BD_JIT && !f32)
-    {
-        CK(cudaEventRecord(im->ev_join, c));
-        CK(cudaStreamWaitEvent(s, im->ev_join, 0));
-        if (timed) CK(cudaEventRecord(e[1], s));
-    }
-    if (!im->BD_JIT)
-    {
-        if (wide)
+        CK(cudaEventRecord(im->ev_fork, s));
+        CK(cudaStreamWaitEvent(c, im->ev_fork, 0));
+        for (size_t L = 0; L + 1 < im->up_beg.size(); L++)
         {
-            const int* nw = im->n_wide;
-            CK(launch_split3(im->d_XS, im->N, im->y0_rows, xs_rows, im->d_XS3, c));   // the skeleton rows y0
-            CK(launch_blk_wide(0, im->d_wide, nw[0], im->d_wseg, im->d_B32, im->d_XS3, xs_rows, im->d_PS, c,
-                               im->d_status));
-            CK(launch_blk_wide(1, im->d_wide + nw[0], nw[1], im->d_wseg, im->d_B32, im->d_XS3, xs_rows, im->d_PS, c,
-                               im->d_status));
-            CK(launch_y1sum(NV, im->d_y1tw, im->n_y1w, im->d_y1_slotsw, im->d_PS, im->d_Y1, im->y0_rows, c));
-            im->st.n_launches += 2;   // the second pass and the split of the inputs
+            int b = im->up_beg[L], n = im->up_beg[L + 1] - b;
+            if (f32) CK(launch_up<float>(NV, im->d_up + b, n, im->d_U32, im->d_XS, c, sweep_tc(im)));
+            else CK(launch_up<double>(NV, im->d_up + b, n, im->d_U64, im->d_XS, c));
         }
-        else if (f32) CK(launch_blk<float>(NV, im->d_blkB, im->n_blkB, im->d_B32, im->d_XS, im->d_PS, c, im->blk_tc, im->d_status,
-                                           im->blk1_small[0][1]));
-        else CK(launch_blk<double>(NV, im->d_blkB, im->n_blkB, im->d_B64, im->d_XS, im->d_PS, c, 0, nullptr,
-                                   im->blk1_small[0][0]));
-        if (!wide) CK(launch_y1sum(NV, im->d_y1t, im->n_y1, im->d_y1_slots, im->d_PS, im->d_Y1, im->y0_rows, c));
-    } else {
-        if (panels) CK(launch_panel_in(NV, im->d_pg, im->n_pg_pts, im->n_pg - im->n_pg_pts, im->d_XS, im->d_pin, c));
-        CK(launch_jit(im->kernel_id, f32, NV, im->d_jtF, im->n_jtF, f32 ? (const void*) im->d_pts32 : (const void*) im->d_pts64,
-                      kparam_of(im), f32 ? 1 : 0, im->jit_tc, im->d_XS, im->d_PS, im->d_Y1, c, im->far_diff ? 0 : 1,
-                      im->d_ppts, im->d_pin, im->d_tiles, im->d_pts32lo, im->d_pplo));
+        if (timed) CK(cudaEventRecord(e[3], c));
+        if (im->BD_JIT && !f32)
+        {
+            CK(cudaEventRecord(im->ev_join, c));
+            CK(cudaStreamWaitEvent(s, im->ev_join, 0));
+            if (timed) CK(cudaEventRecord(e[1], s));
+        }
+        if (!im->BD_JIT)
+        {
+            if (wide)
+            {
+                const int* nw = im->n_wide;
+                CK(launch_split3(im->d_XS, im->N, im->y0_rows, xs_rows, im->d_XS3, c));   // the skeleton rows y0
+                CK(launch_blk_wide(0, im->d_wide, nw[0], im->d_wseg, im->d_B32, im->d_XS3, xs_rows, im->d_PS, c,
+                                   im->d_status));
+                CK(launch_blk_wide(1, im->d_wide + nw[0], nw[1], im->d_wseg, im->d_B32, im->d_XS3, xs_rows, im->d_PS, c,
+                                   im->d_status));
+                CK(launch_y1sum(NV, im->d_y1tw, im->n_y1w, im->d_y1_slotsw, im->d_PS, im->d_Y1, im->y0_rows, c));
+                im->st.n_launches += 2;   // the second pass and the split of the inputs
+            }
+            else if (f32) CK(launch_blk<float>(NV, im->d_blkB, im->n_blkB, im->d_B32, im->d_XS, im->d_PS, c, im->blk_tc, im->d_status,
+                                               im->blk1_small[0][1]));
+            else CK(launch_blk<double>(NV, im->d_blkB, im->n_blkB, im->d_B64, im->d_XS, im->d_PS, c, 0, nullptr,
+                                       im->blk1_small[0][0]));
+            if (!wide) CK(launch_y1sum(NV, im->d_y1t, im->n_y1, im->d_y1_slots, im->d_PS, im->d_Y1, im->y0_rows, c));
+        } else {
+            if (panels) CK(launch_panel_in(NV, im->d_pg, im->n_pg_pts, im->n_pg - im->n_pg_pts, im->d_XS, im->d_pin, c));
+            CK(launch_jit(im->kernel_id, f32, NV, im->d_jtF, im->n_jtF, f32 ? (const void*) im->d_pts32 : (const void*) im->d_pts64,
+                          kparam_of(im), f32 ? 1 : 0, im->jit_tc, im->d_XS, im->d_PS, im->d_Y1, c, im->far_diff ? 0 : 1,
+                          im->d_ppts, im->d_pin, im->d_tiles, im->d_pts32lo, im->d_pplo));
+        }
+        if (timed) CK(cudaEventRecord(e[4], c));
+        for (size_t L = 0; L + 1 < im->dn_beg.size(); L++)
+        {
+            int b = im->dn_beg[L], n = im->dn_beg[L + 1] - b;
+            if (f32) CK(launch_down<float>(NV, im->d_dn + b, n, im->d_U32, im->d_Y1, im->d_PS, im->d_PUSH, c, sweep_tc(im)));
+            else CK(launch_down<double>(NV, im->d_dn + b, n, im->d_U64, im->d_Y1, im->d_PS, im->d_PUSH, c));
+        }
+        if (timed) CK(cudaEventRecord(e[5], c));
+        CK(cudaEventRecord(im->ev_join, c));
     }
-    if (timed) CK(cudaEventRecord(e[4], c));
-    for (size_t L = 0; L + 1 < im->dn_beg.size(); L++)
-    {
-        int b = im->dn_beg[L], n = im->dn_beg[L + 1] - b;
-        if (f32) CK(launch_down<float>(NV, im->d_dn + b, n, im->d_U32, im->d_Y1, im->d_PS, im->d_PUSH, c, sweep_tc(im)));
-        else CK(launch_down<double>(NV, im->d_dn + b, n, im->d_U64, im->d_Y1, im->d_PS, im->d_PUSH, c));
-    }
-    if (timed) CK(cudaEventRecord(e[5], c));
-    CK(cudaEventRecord(im->ev_join, c));
     // the near field, on the caller's stream
     if (!im->BD_JIT)
     {
@@ -2088,7 +2094,7 @@ int run_panel(h2gpu_image* im, int NV, int nv, const double* X, long long x_rs, 
         im->st.n_launches += panels ? 2 : 0;
     }
     if (timed) CK(cudaEventRecord(e[2], s));
-    CK(cudaStreamWaitEvent(s, im->ev_join, 0));
+    if (has_chain(im)) CK(cudaStreamWaitEvent(s, im->ev_join, 0));
     if (wide) CK(launch_asm(NV, im->d_asmw, im->n_asmw, im->d_asm_slotsw, im->d_PS, im->d_fwd, Y, y_rs, y_cs, nv, im->N, s));
     else CK(launch_asm(NV, im->d_asm, im->n_asm, im->d_asm_slots, im->d_PS, im->d_fwd, Y, y_rs, y_cs, nv, im->N, s));
     if (timed && uses_status(im, NV))
@@ -2220,11 +2226,18 @@ int apply_device(h2gpu_image* im, int n_vec, const double* X, long long x_rs, lo
             return t;
         };
         const bool after_up = im->BD_JIT && im->precision == H2GPU_PREC_FP64;   // D's start: run_panel
-        ph[0] += pair ? ms(0, 1) + ms(2, 3) : after_up ? ms(0, 3) : ms(0, 1) + ms(1, 3);   // gather + upward
-        ph[1] += ms(3, 4);                         // B
-        ph[2] += ms(4, 5);                         // downward
+        const bool chain = pair || has_chain(im);
         ph[3] += ms(1, 2);                         // D
-        ph[4] += std::min(ms(5, 6), ms(2, 6));     // assemble
+        if (chain)
+        {
+            ph[0] += pair ? ms(0, 1) + ms(2, 3) : after_up ? ms(0, 3) : ms(0, 1) + ms(1, 3);   // gather + upward
+            ph[1] += ms(3, 4);                     // B
+            ph[2] += ms(4, 5);                     // downward
+            ph[4] += std::min(ms(5, 6), ms(2, 6)); // assemble
+        } else {
+            ph[0] += ms(0, 1);
+            ph[4] += ms(2, 6);
+        }
         total += ms(0, 6);
     }
     for (int k = 0; k < 5; k++) im->st.ms_phase[k] += ph[k];
