@@ -20,8 +20,7 @@
 // Layout.  Q is kept explicitly (m x m per node, stored as Q^T row-major, i.e. row r
 // = column r of Q), formed once from the reflectors at create by k_ulv_form_q, so
 // that Q^T b and Q b are plain products instead of a chain of k dependent reflector
-// steps; L as H2Pack stores it (m x m row-major).  Rows have an even stride and start so
-// that Q's rows and the columns from Ls on are 16-byte aligned; the padding is zero.
+// steps; L as H2Pack stores it (m x m row-major).
 // FP64 throughout; every sum has a fixed order, so results are deterministic.
 #include <algorithm>
 #include <cmath>
@@ -51,13 +50,13 @@ constexpr unsigned kFull = 0xffffffffu;
 constexpr int kPollLimit = 1 << 22;        // polls (a few seconds) before a wait gives up
 
 struct UlvNode {
-    long long q_off;     // Q^T (m rows of stride q_ld) in the Q arena; -1: no Q
-    long long l_off;     // L (m rows of stride l_ld) in the L arena
+    long long q_off;     // Q^T (m x m row-major) in the Q arena; -1: no Q
+    long long l_off;     // L (m x m row-major) in the L arena
     long long idx_off;   // m indices into the permuted vector, m entries of the tagged vectors
     long long p_off;     // LU: m - I pivots; -1: none
     long long d_off;     // inverses of the diagonal blocks of the triangular factor (64 x 64
                          // row-major each); LU: of L0, then of U0
-    int m, I, q_ld, l_ld;
+    int m, I, pad0, pad1;
 };
 
 // diagonal block at (I + at, I + at) of a node's factor, its inverse at d_off
@@ -70,7 +69,7 @@ struct UlvQJob {
     long long v_off;     // k reflectors of length m, reflector j at v + j m (1 at j,
                          // zeros above), then tau (k entries)
     long long q_off;
-    int m, k, ld, pad1;
+    int m, k, pad0, pad1;
 };
 
 enum { CH_UP = 0, CH_DOWN = 1, LU_UP = 2, LU_DOWN = 3 };
@@ -225,21 +224,26 @@ __device__ __forceinline__ void rows_product(const double* __restrict__ A, int l
     }
 }
 
-// acc += sum_r A[r][c] x[r] over the 64-row tiles t0, t0 + dt, .. of nr rows, c = 2 lane and
-// 2 lane + 1 of nc columns: a warp takes eight rows of a tile (in two halves), its lanes
-// the columns
+// acc += sum_r A[r][c] x[r] over the 64-row tiles t0, t0 + dt, .. of nr rows, c = lane and
+// lane + 32 of nc columns: a warp takes eight rows of a tile (in two halves), its lanes the
+// columns
 template <typename IN>
 __device__ __forceinline__ void cols_product(const double* __restrict__ A, int ld, int nr, int nc, int t0, int dt,
                                              int cnt, const IN& in, double2& acc)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const double* const a = A + (2 * lane < nc ? 2 * lane : 0);
+    const bool c0 = lane < nc, c1 = lane + 32 < nc;
+    const double* const a = A + (c0 ? lane : 0);
     double2 u[4], v[4];
     typename IN::R q{};
     auto fetch = [&](int r0, double2 (&b)[4]) {
 #pragma unroll
         for (int k = 0; k < 4; k++)
-            b[k] = r0 + k < nr ? __ldg(reinterpret_cast<const double2*>(a + (long long) (r0 + k) * ld)) : make_double2(0.0, 0.0);
+        {
+            const double* const p = a + (long long) (r0 + k) * ld;
+            b[k].x = r0 + k < nr ? __ldg(p) : 0.0;
+            b[k].y = r0 + k < nr && c1 ? __ldg(p + 32) : 0.0;
+        }
     };
     auto start = [&](int r) {
         if (r < nr) q = in.issue(r);
@@ -359,7 +363,7 @@ __global__ void __launch_bounds__(kUT, 2) k_ulv_units(const UlvNode* __restrict_
         const int m = N.m, I = N.I, n2 = m - I, at = un.at;
         const int* const idx = idxs + N.idx_off;
         const double* const L = Lf + N.l_off;
-        const double* const T = L + (long long) I * N.l_ld + I;
+        const double* const T = L + (long long) I * m + I;
         Tagged* const w = W + N.idx_off;
         Tagged* const x = X + N.idx_off;
         const bool hasq = N.q_off >= 0;
@@ -370,7 +374,7 @@ __global__ void __launch_bounds__(kUT, 2) k_ulv_units(const UlvNode* __restrict_
             __syncthreads();
             const int nr = min(kB, m - at);
             double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-            rows_product(Qt + N.q_off + (long long) at * N.q_ld, N.q_ld, nr, m, 0, 1, (m + kB - 1) / kB, InShared{sx}, acc);
+            rows_product(Qt + N.q_off + (long long) at * m, m, nr, m, 0, 1, (m + kB - 1) / kB, InShared{sx}, acc);
             rows_reduce(acc, sr);
             __syncwarp();
             if (lane < 8 && 8 * warp + lane < nr) tag_put(w + at + 8 * warp + lane, sr[8 * warp + lane]);
@@ -389,7 +393,7 @@ __global__ void __launch_bounds__(kUT, 2) k_ulv_units(const UlvNode* __restrict_
                 const int i = e / kB, j = e % kB;      // row, column of the factor block
                 double v = 0.0;
                 if (MODE == LU_DOWN ? j >= i : j < i || (MODE != LU_UP && j == i))
-                    if (i < nr && j < nr) v = __ldg(T + (long long) (at + i) * N.l_ld + at + j);
+                    if (i < nr && j < nr) v = __ldg(T + (long long) (at + i) * m + at + j);
                 if (i == j && (MODE == LU_UP || i >= nr)) v = 1.0;
                 const int k = MODE == CH_DOWN ? i * kDS + j : j * kDS + i;
                 sD[k] = v;
@@ -409,20 +413,20 @@ __global__ void __launch_bounds__(kUT, 2) k_ulv_units(const UlvNode* __restrict_
             double2 ac = make_double2(0.0, 0.0);
             const InTagged xs{x + I, status};
             if constexpr (UP)
-                rows_product(T + (long long) at * N.l_ld, N.l_ld, nr, n2, 0, 1, at / kB, xs, acc);
+                rows_product(T + (long long) at * m, m, nr, n2, 0, 1, at / kB, xs, acc);
             else if constexpr (MODE == LU_DOWN)
             {
-                rows_product(L + (long long) (I + at) * N.l_ld, N.l_ld, nr, I, 0, 1, (I + kB - 1) / kB,
+                rows_product(L + (long long) (I + at) * m, m, nr, I, 0, 1, (I + kB - 1) / kB,
                              InIndexed{px, idx}, acc);
-                rows_product(T + (long long) at * N.l_ld, N.l_ld, nr, n2, nt - 1, -1, after, xs, acc);
+                rows_product(T + (long long) at * m, m, nr, n2, nt - 1, -1, after, xs, acc);
             } else {
-                cols_product(L + I + at, N.l_ld, I, nr, 0, 1, (I + kB - 1) / kB, InIndexed{px, idx}, ac);
-                cols_product(T + at, N.l_ld, n2, nr, nt - 1, -1, after, xs, ac);
+                cols_product(L + I + at, m, I, nr, 0, 1, (I + kB - 1) / kB, InIndexed{px, idx}, ac);
+                cols_product(T + at, m, n2, nr, nt - 1, -1, after, xs, ac);
             }
             if constexpr (MODE == CH_DOWN)
             {
-                sP[warp * kB + 2 * lane] = ac.x;
-                sP[warp * kB + 2 * lane + 1] = ac.y;
+                sP[warp * kB + lane] = ac.x;
+                sP[warp * kB + lane + 32] = ac.y;
             } else rows_reduce(acc, sP);
             __syncthreads();
             if (tid < kB)
@@ -459,7 +463,7 @@ __global__ void __launch_bounds__(kUT, 2) k_ulv_units(const UlvNode* __restrict_
             double b = 0.0;
             if (tid < nr) b = hasq ? tag_wait(w + at + tid, tag_get(w + at + tid), status) : px[idx[at + tid]];
             double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-            rows_product(L + (long long) at * N.l_ld + I, N.l_ld, nr, n2, 0, 1, (n2 + kB - 1) / kB, InTagged{x + I, status}, acc);
+            rows_product(L + (long long) at * m + I, m, nr, n2, 0, 1, (n2 + kB - 1) / kB, InTagged{x + I, status}, acc);
             rows_reduce(acc, sP);
             __syncthreads();
             if (tid < nr)
@@ -475,9 +479,9 @@ __global__ void __launch_bounds__(kUT, 2) k_ulv_units(const UlvNode* __restrict_
             __syncthreads();
             const int nc = min(kB, m - at);
             double2 ac = make_double2(0.0, 0.0);
-            cols_product(Qt + N.q_off + at, N.q_ld, m, nc, 0, 1, (m + kB - 1) / kB, InShared{sx}, ac);
-            sP[warp * kB + 2 * lane] = ac.x;
-            sP[warp * kB + 2 * lane + 1] = ac.y;
+            cols_product(Qt + N.q_off + at, m, m, nc, 0, 1, (m + kB - 1) / kB, InShared{sx}, ac);
+            sP[warp * kB + lane] = ac.x;
+            sP[warp * kB + lane + 32] = ac.y;
             __syncthreads();
             if (tid < nc)
             {
@@ -514,7 +518,7 @@ __global__ void __launch_bounds__(kUT) k_ulv_form_q(const UlvQJob* __restrict__ 
     const int c = blockIdx.x * kUW + warp;
     if (c >= J.m) return;
     const int m = J.m;
-    double* const x = Qt + J.q_off + (long long) c * J.ld;
+    double* const x = Qt + J.q_off + (long long) c * m;
     for (int i = lane; i < m; i += 32) x[i] = i == c ? 1.0 : 0.0;
     __syncwarp();
     const double* const v = V + J.v_off;
@@ -541,8 +545,8 @@ __global__ void __launch_bounds__(kB) k_ulv_diag(const UlvDiagJob* __restrict__ 
     const UlvDiagJob J = jobs[blockIdx.x];
     const UlvNode N = nodes[J.node];
     const int nr = min(kB, N.m - N.I - J.at), c = threadIdx.x;
-    const double* const T = Lf + N.l_off + (long long) (N.I + J.at) * N.l_ld + N.I + J.at;
-    for (int i = 0; i < kB; i++) sD[i * kB + c] = i < nr && c < nr ? T[(long long) i * N.l_ld + c] : (i == c ? 1.0 : 0.0);
+    const double* const T = Lf + N.l_off + (long long) (N.I + J.at) * N.m + N.I + J.at;
+    for (int i = 0; i < kB; i++) sD[i * kB + c] = i < nr && c < nr ? T[(long long) i * N.m + c] : (i == c ? 1.0 : 0.0);
     __syncthreads();
     for (int t = 0; t < kB; t++)
     {
@@ -755,11 +759,7 @@ H2G_API int h2gpu_ulv_create(const h2gpu_ulv_desc* d, h2gpu_ulv** out)
                 return ulv_fail(H2GPU_ERR_INVALID, "node %d: index %d out of range", node, d->idx[node][i]);
         UlvNode& N = nodes[node];
         N.m = m; N.I = I;
-        // an even row stride with room for one element past the row, and columns I .. of
-        // every row on an even element
-        N.l_ld = (m + 2) & ~1; N.q_ld = (m + 1) & ~1;
-        nl += nl & 1;
-        N.l_off = nl + (I & 1); nl += (long long) m * N.l_ld + 2;
+        N.l_off = nl; nl += (long long) m * m;
         N.idx_off = ni; ni += m;
         N.d_off = nd;
         for (int up = 0; up <= (d->lu ? 1 : 0); up++)
@@ -771,9 +771,9 @@ H2G_API int h2gpu_ulv_create(const h2gpu_ulv_desc* d, h2gpu_ulv** out)
         {
             if (k > m) return ulv_fail(H2GPU_ERR_UNSUPPORTED, "node %d: %d reflectors of length %d", node, k, m);
             if (!d->Q[node]) return ulv_fail(H2GPU_ERR_INVALID, "node %d: Q missing", node);
-            N.q_off = nq; nq += (long long) m * N.q_ld;
+            N.q_off = nq; nq += (long long) m * m;
             q_cap = std::max(q_cap, m);
-            jobs.push_back(UlvQJob{nv, N.q_off, m, k, N.q_ld, 0});
+            jobs.push_back(UlvQJob{nv, N.q_off, m, k, 0, 0});
             nv += (long long) k * m + k;
         }
         if (d->lu)
@@ -855,9 +855,6 @@ H2G_API int h2gpu_ulv_create(const h2gpu_ulv_desc* d, h2gpu_ulv** out)
         step(cudaMemcpy(u->d_nodes, nodes.data(), sizeof(UlvNode) * nodes.size(), cudaMemcpyHostToDevice), "upload") &&
         step(cudaMemcpy(u->d_units, units.data(), sizeof(UlvUnit) * units.size(), cudaMemcpyHostToDevice), "upload") &&
         step(cudaHostAlloc((void**) &u->h_status, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped), "status word") &&
-        // the padding of the factors is read (times zero or beside the row)
-        step(cudaMemset(u->d_Q, 0, std::max<size_t>(8 * (size_t) nq, 16)), "clearing") &&
-        step(cudaMemset(u->d_L, 0, std::max<size_t>(8 * (size_t) nl, 16)), "clearing") &&
         step(cudaMemcpy(u->d_idx, hidx.data(), 4 * (size_t) ni, cudaMemcpyHostToDevice), "upload") &&
         step(np ? cudaMemcpy(u->d_p, hp.data(), 4 * (size_t) np, cudaMemcpyHostToDevice) : cudaSuccess, "upload") &&
         step(cudaMemcpy(u->d_fwd, d->fwd_pmt_idx, 4 * (size_t) n, cudaMemcpyHostToDevice), "upload") &&
@@ -868,7 +865,7 @@ H2G_API int h2gpu_ulv_create(const h2gpu_ulv_desc* d, h2gpu_ulv** out)
         {
             const UlvNode& N = nodes[node];
             if (N.m == 0) continue;
-            if (!step(cudaMemcpy2D(u->d_L + N.l_off, 8 * (size_t) N.l_ld, d->L[node], 8 * (size_t) d->l_ld[node],
+            if (!step(cudaMemcpy2D(u->d_L + N.l_off, 8 * (size_t) N.m, d->L[node], 8 * (size_t) d->l_ld[node],
                                    8 * (size_t) N.m, (size_t) N.m, cudaMemcpyHostToDevice), "factor upload"))
                 break;
         }
