@@ -5,7 +5,8 @@
 //   k_gather      forward permutation of the input panel into XS          (matvec.c:1174-1179)
 //   k_up          upward sweep y0 = U^T x, one CTA per node                 (matvec.c:95-177)
 //   k_blk         stored B / D block chunks, one read feeds A*v and A^T*w  (matvec.c:303-437, 864-998)
-//   k_jit         on-the-fly B / D kernel blocks, owner computes           (matvec.c:586-764, 1002-1145)
+//   k_jit*        on-the-fly B / D kernel blocks, owner computes           (matvec.c:586-764, 1002-1145)
+//                 (k_jit64 FP64; FP32: k_jit_tc panels of 8 / 16, k_jit2 narrower, k_jit RPY)
 //   k_down        downward sweep U * y1 with slot sums and push-down       (matvec.c:767-861)
 //   k_asm         sum of a leaf's partial slots + backward permutation     (matvec.c:1251-1278)
 //   k_direct      FP64 direct sum (examples/direct_nbody.h:2-54)
