@@ -67,6 +67,9 @@ static int fail(int code, const char* fmt, ...)
         if (s_ != H2GPU_OK) return s_;   \
     } while (0)
 
+// work space of h2gpu_matvec_device_noalloc
+#define H2GPU_NOALLOC_SCRATCH_DOUBLES (2u * 1024u * 1024u)
+
 namespace {
 
 template <typename T>
@@ -568,7 +571,19 @@ int build_plan(h2gpu_image* im, const h2gpu_desc* d, HostPlan& hp)
             im->bmap[0].push_back({(long long) d->B_ptr[i], off32B[i], d->B_nrow[i], d->B_ncol[i]});
         for (int i = 0; i < d->n_D; i++)
             im->bmap[1].push_back({(long long) d->D_ptr[i], off32D[i], d->D_nrow[i], d->D_ncol[i]});
-        const int RB_B = task_rows(d->n_B, d->B_nrow, d->B_ncol), RB_D = task_rows(d->n_D, d->D_nrow, d->D_ncol);
+        int RB_B = task_rows(d->n_B, d->B_nrow, d->B_ncol), RB_D = task_rows(d->n_D, d->D_nrow, d->D_ncol);
+        // Smaller tasks have more slots (a few hundred blocks of thousands of columns: several
+        // times as many): not where h2gpu_matvec_device_noalloc's work space might not hold them
+        auto slot_rows = [&](int n, const int* nrow, const int* ncol, int RB) {
+            long long rows = 0;
+            for (int i = 0; i < n; i++)
+                if (nrow[i] > 0 && ncol[i] > 0)
+                    rows += nrow[i] + (long long) ncol[i] * ((nrow[i] + rows_per_task(nrow[i], RB) - 1) / rows_per_task(nrow[i], RB));
+            return rows;
+        };
+        if (N + 3 * im->y0_rows + ps + slot_rows(d->n_B, d->B_nrow, d->B_ncol, RB_B) +
+                slot_rows(d->n_D, d->D_nrow, d->D_ncol, RB_D) > (long long) H2GPU_NOALLOC_SCRATCH_DOUBLES)
+            RB_B = RB_D = 1024;
         for (int i = 0; i < d->n_B; i++)
         {
             int n0 = d->r_adm_pairs[2 * i], n1 = d->r_adm_pairs[2 * i + 1];
@@ -2944,8 +2959,6 @@ H2G_API int h2gpu_pp_sketch_id(int kernel_id, const double* krnl_param, int n_kr
 // allocating apply (h2gpu_matvec, h2gpu_matmul, h2gpu_matmul_device) creates; until
 // then this entry point refuses it with H2GPU_ERR_STATE.  The caller's current device
 // is left as it was.
-
-#define H2GPU_NOALLOC_SCRATCH_DOUBLES (2u * 1024u * 1024u)
 
 static __device__ __align__(256) double g_noalloc_scratch[H2GPU_NOALLOC_SCRATCH_DOUBLES];
 

@@ -36,3 +36,20 @@ def test_matches_64_bit_product(kernel, n, leaf, precision):
         for nv in (2, 17):
             assert np.linalg.norm(img.matmul(Xh[:, :nv], layout) - Yh[:, :nv]) < tol * np.linalg.norm(Yh[:, :nv])
     img.close()
+
+
+def test_few_large_blocks_fit_the_no_allocation_apply():
+    """36 near blocks of 3,000 columns: tasks small enough to fill the GPU would have 2.6 million
+    slots, past that apply's work space; such an image keeps its tall tasks (same sums in another
+    order, 1e-13)."""
+    import torch
+    from perf import cases
+    case = {"kind": "apply", "kernel": "coulomb", "n": 24000, "leaf": 8000, "mode": "generate", "precision": "fp64", "api": "device"}
+    rep = cases.Rep(case, 24000, 4)
+    img = cases.Image(rep.describe(), "fp64", blocks="generate")
+    x = cases._rhs(case, 24000, 1, 4)[:, 0].contiguous()
+    y0, y = img.matmul_device(x[:, None].contiguous())[:, 0], torch.empty_like(x)
+    img.matvec_device_noalloc(x, y)
+    torch.cuda.synchronize()
+    assert float((y - y0).norm() / y0.norm()) < 1e-13
+    img.close()
