@@ -682,6 +682,11 @@ int enqueue_solve(h2gpu_ulv* u, int op, const double* d_b, double* d_x, cudaStre
     return cuda_status(cudaGetLastError(), "solve launch");
 }
 
+// cudaMemcpy from pageable memory may return once the data is staged, with the transfer itself
+// still on its way in the legacy stream, which the object's non-blocking stream does not wait
+// for: kernels on that stream read uploads after this only.
+cudaError_t uploads_landed() { return cudaStreamSynchronize(cudaStreamLegacy); }
+
 // Units of one level of a sweep, in an order in which every unit depends on earlier ones
 // only; the triangular chains of a level's nodes advance side by side.
 void level_units(const std::vector<UlvNode>& nodes, const int* list, int cnt, bool up, bool lu, std::vector<UlvUnit>& out)
@@ -872,6 +877,7 @@ H2G_API int h2gpu_ulv_create(const h2gpu_ulv_desc* d, h2gpu_ulv** out)
     }
     if (st == H2GPU_OK && !djobs.empty() && step(cudaMalloc(&d_djobs, sizeof(UlvDiagJob) * djobs.size()), "diagonal blocks") &&
         step(cudaMemcpy(d_djobs, djobs.data(), sizeof(UlvDiagJob) * djobs.size(), cudaMemcpyHostToDevice), "diagonal blocks") &&
+        step(uploads_landed(), "diagonal blocks") &&
         step(cudaFuncSetAttribute(k_ulv_diag, cudaFuncAttributeMaxDynamicSharedMemorySize, 16 * kB * kB), "diagonal blocks"))
     {
         k_ulv_diag<<<(unsigned) djobs.size(), kB, 16 * kB * kB, u->stream>>>(d_djobs, u->d_nodes, u->d_L, u->d_D);
@@ -881,7 +887,8 @@ H2G_API int h2gpu_ulv_create(const h2gpu_ulv_desc* d, h2gpu_ulv** out)
     if (st == H2GPU_OK && !jobs.empty() && step(cudaMalloc(&d_v, 8 * (size_t) nv), "reflector staging") &&
         step(cudaMalloc(&d_jobs, sizeof(UlvQJob) * jobs.size()), "reflector staging") &&
         step(cudaMemcpy(d_v, hv.data(), 8 * (size_t) nv, cudaMemcpyHostToDevice), "reflector upload") &&
-        step(cudaMemcpy(d_jobs, jobs.data(), sizeof(UlvQJob) * jobs.size(), cudaMemcpyHostToDevice), "reflector upload"))
+        step(cudaMemcpy(d_jobs, jobs.data(), sizeof(UlvQJob) * jobs.size(), cudaMemcpyHostToDevice), "reflector upload") &&
+        step(uploads_landed(), "reflector upload"))
     {
         int mq = 1;
         for (const UlvQJob& J : jobs) mq = std::max(mq, J.m);
@@ -896,6 +903,8 @@ H2G_API int h2gpu_ulv_create(const h2gpu_ulv_desc* d, h2gpu_ulv** out)
     if (d_v) cudaFree(d_v);
     if (d_jobs) cudaFree(d_jobs);
     if (d_djobs) cudaFree(d_djobs);
+    // the first solve may come on any stream (no diagonal block and no reflector: nothing has waited yet)
+    step(uploads_landed(), "upload");
     if (st == H2GPU_OK)
     {
         // The limit is a per-function setting of the process: it is set to the device's

@@ -45,3 +45,42 @@ def test_an_infinite_entry_reaches_only_what_depends_on_it():
     order[inv] = torch.arange(150, device="cuda")          # x[i] = permuted[bwd[i]]
     assert torch.equal(clean[order][:k], bad[order][:k])
     assert not torch.isfinite(bad[order][k:]).all()
+
+
+class _Kept:
+    """The factors of one case, with the host arrays that create read kept for the test."""
+
+    def __new__(cls, case, seed, change=None):
+        from perf import cases
+
+        class Ulv(cases._Ulv):
+            def __setattr__(self, k, v):
+                if not (k in ("hQ", "hL") and v is None):
+                    super().__setattr__(k, v)
+
+        u = Ulv(case, seed)
+        if change:
+            change(u)
+        return u
+
+
+@pytest.mark.parametrize("lu", [False, True])
+def test_a_solve_right_after_create_sees_whole_factors(lu):
+    """One node of 72 MB and three levels of small ones; the caller's arrays are overwritten as
+    soon as create returns, and the first solve starts at once on the object's own stream."""
+    import numpy as np
+    import torch
+    from h2pack_b200.h2pack import _dptr
+    from perf import cases
+    for n, leaf in ((3000, 3000), (3003, 60)):
+        case = {"kind": "ulv", "n": n, "leaf": leaf, "frac": 0.6, "frac_up": 0.5, "lu": lu, "op": 3}
+        b = np.random.default_rng(n).standard_normal(n)
+        e = cases._Ulv(case, 8).solve(3, torch.from_numpy(b).cuda()).cpu().numpy()
+        u = _Kept(case, 8)
+        torch.cuda.synchronize()
+        u.create()
+        for a in u.hQ + u.hL:
+            a.fill(np.nan)
+        x = np.empty(n)
+        assert u.lib.h2gpu_ulv_solve(u.handle, 3, _dptr(b), _dptr(x)) == 0
+        assert np.linalg.norm(x - e) < 1e-13 * np.linalg.norm(e), (n, lu)
