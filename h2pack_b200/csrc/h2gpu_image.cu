@@ -83,6 +83,11 @@ int upload(const std::vector<T>& h, T** d, size_t& total)
     return H2GPU_OK;
 }
 
+// cudaMemcpy from pageable memory may return once the data is staged, with the transfer itself
+// still on its way in the legacy stream, which the image's non-blocking streams do not wait
+// for: kernels on those read uploads after this only.
+cudaError_t uploads_landed() { return cudaStreamSynchronize(cudaStreamLegacy); }
+
 struct Ev {
     cudaEvent_t e[8] = {};
 };
@@ -1809,6 +1814,7 @@ int upload_plan(h2gpu_image* im, const h2gpu_desc* d, HostPlan& hp)
     if (im->n_pg > 0 && d->krnl_dim == 1)
     {
         // the point half of the panels is static
+        CK(uploads_landed());
         CK(cudaMalloc(&im->d_ppts, sizeof(float4) * 8 * (size_t) im->n_pg));
         im->bytes += sizeof(float4) * 8 * (size_t) im->n_pg;
         CK(launch_panel_pts(im->d_pg, im->n_pg, im->d_pts32, kparam_of(im).sigma, im->d_ppts, im->stream));
@@ -2130,6 +2136,7 @@ int check_status(h2gpu_image* im)
     {
         *im->h_status = 0;
         CK(cudaMemset(im->d_status, 0, sizeof(int)));
+        CK(uploads_landed());
         return fail(H2GPU_ERR_DEVICE, "tcgen05 block kernel: a bounded wait on the MMA completion expired");
     }
     return H2GPU_OK;
@@ -2168,6 +2175,7 @@ int generate_blocks(h2gpu_image* im, const GenPlan& g)
         // the FP32 rows' padding stays zero (the kernels read it through 16-byte loads)
         if (fp32 && nB) e = cudaMemsetAsync(B, 0, es * nB, im->stream);
         if (fp32 && nD && e == cudaSuccess) e = cudaMemsetAsync(D, 0, es * nD, im->stream);
+        if (e == cudaSuccess) e = uploads_landed();
         const KParam kp = kparam_of(im);
         // one launch per block kind, in slices that keep the grid inside its limits
         const int tB = (int) g.tB.size(), tD = (int) g.tD.size();
@@ -2414,6 +2422,7 @@ H2G_API int h2gpu_image_create(const h2gpu_desc* desc, const h2gpu_options* opt,
                                cudaHostAlloc(&im->h_status, sizeof(int), cudaHostAllocDefault) != cudaSuccess))
             st = fail(H2GPU_ERR_NOMEM, "status word allocation failed");
         if (st == H2GPU_OK) *im->h_status = 0;
+        if (st == H2GPU_OK && uploads_landed() != cudaSuccess) st = fail(H2GPU_ERR_CUDA, "upload failed");
     } while (0);
     if (st != H2GPU_OK)
     {

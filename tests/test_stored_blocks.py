@@ -53,3 +53,25 @@ def test_few_large_blocks_fit_the_no_allocation_apply():
     torch.cuda.synchronize()
     assert float((y - y0).norm() / y0.norm()) < 1e-13
     img.close()
+
+
+@pytest.mark.parametrize("kernel,n,leaf,mode", [("coulomb", 6000, 300, "given"), ("coulomb", 6000, 300, "generate"),
+                                                ("gaussian", 20000, 400, "jit")])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_an_apply_right_after_create_sees_whole_uploads(kernel, n, leaf, mode, precision):
+    """The caller's arrays are overwritten as soon as create returns, and the first apply starts at
+    once on the image's own stream."""
+    import numpy as np
+    import torch
+    from perf import cases
+    case = {"kind": "apply", "kernel": kernel, "n": n, "leaf": leaf, "mode": mode, "precision": precision, "api": "host"}
+    rep = cases.Rep(case, n, 6)
+    X = cases._rhs(case, n, 8, 6)
+    Y, Xh = rep.apply(X).cpu().numpy(), X.cpu().numpy()
+    d = rep.describe(mode == "given")
+    torch.cuda.synchronize()
+    img = cases.Image(d, precision, blocks="generate" if mode == "generate" else "given")
+    for a in rep.host.values():
+        a.fill(np.nan if a.dtype == np.float64 else 0)
+    assert np.linalg.norm(img.matmul(Xh) - Y) < (1e-13 if precision == "fp64" else 2e-6) * np.linalg.norm(Y)
+    img.close()
