@@ -48,6 +48,10 @@ constexpr int kDS = kB + 4;                // column stride of a diagonal block 
 constexpr int kMaxNodeRows = 13872;        // larger nodes are refused
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kPollLimit = 1 << 22;        // polls (a few seconds) before a wait gives up
+// Largest || |M| |M^-1| || of a diagonal block M that is solved with its inverse E.  One step of
+// refinement leaves a residual of about (128 u || |M| |E| ||)^2 of the block's right-hand
+// side beside the rounding that substitution has too (u = 2^-53): 2e-18 at this bound.
+constexpr double kInverseMax = 1e5;
 
 struct UlvNode {
     long long q_off;     // Q^T (m x m row-major) in the Q arena; -1: no Q
@@ -55,7 +59,8 @@ struct UlvNode {
     long long idx_off;   // m indices into the permuted vector, m entries of the tagged vectors
     long long p_off;     // LU: m - I pivots; -1: none
     long long d_off;     // inverses of the diagonal blocks of the triangular factor (64 x 64
-                         // row-major each); LU: of L0, then of U0
+                         // row-major each); LU: of L0, then of U0.  Block at d_off + k 64^2 has
+                         // its flag at index d_off / 64^2 + k: 1 is solved by substitution
     int m, I, pad0, pad1;
 };
 
@@ -321,6 +326,23 @@ __device__ __forceinline__ double apply_diag(const double* s, const double* r)
     return a[0];
 }
 
+// x = M^-1 r by substitution, one warp, M as apply_diag has it: lane owns rows lane and lane + 32
+template <bool LOWER>
+__device__ __forceinline__ void substitute(const double* s, const double* r, double* x)
+{
+    const int lane = threadIdx.x & 31;
+    double r0 = r[lane], r1 = r[lane + 32];
+#pragma unroll 1
+    for (int t = 0; t < kB; t++)
+    {
+        const int j = LOWER ? t : kB - 1 - t;
+        const double v = __shfl_sync(kFull, j < 32 ? r0 : r1, j & 31) / s[j * kDS + j];
+        if (lane == 0) x[j] = v;
+        if (LOWER ? lane > j : lane < j) r0 = fma(-s[j * kDS + lane], v, r0);
+        if (LOWER ? lane + 32 > j : lane + 32 < j) r1 = fma(-s[j * kDS + lane + 32], v, r1);
+    }
+}
+
 // The units of one level of one sweep.  What bounds it: the factors are read once a sweep
 // (HBM), and the triangular solve of a node is a chain of (m - I) / 64 dependent steps:
 // publish a block's 64 entries, read them on another SM through L2, the product with the
@@ -328,8 +350,8 @@ __device__ __forceinline__ double apply_diag(const double* s, const double* r)
 // block.  A block is solved with its inverse (made at create) and one step of refinement
 // against the block itself, three 64 x 64 products, about 0.5 us; substitution by one warp
 // (64 dependent shuffle / multiply-add steps) measured 2.15 ms for the solve below, the
-// inverse 1.26 ms, with the smaller error of the two (3.49e-15 and 3.51e-15 from the
-// 64-bit solve).
+// inverse 1.26 ms (3.49e-15 and 3.51e-15 from the 64-bit solve).  That is sound for blocks
+// whose inverse is (kInverseMax); the others, which k_ulv_diag flags, are solved by substitution.
 // One CTA per node (the earlier form) read the root's 471 MB through one SM.  HSS tree of
 // N = 20,000 with 64 leaves, root of 7,700 rows, Cholesky, op 3: 36.8 -> 1.26 ms (2.3 GB of
 // factors, 0.36 ms at the copy bandwidth).
@@ -338,6 +360,7 @@ __global__ void __launch_bounds__(kUT, 2) k_ulv_units(const UlvNode* __restrict_
                                                       const UlvUnit* __restrict__ units, int n_units, int* ticket,
                                                       int q_cap, const double* __restrict__ Qt,
                                                       const double* __restrict__ Lf, const double* __restrict__ Dinv,
+                                                      const unsigned char* __restrict__ subst,
                                                       const int* __restrict__ idxs, const int* __restrict__ piv,
                                                       double* px, Tagged* W, Tagged* X,
                                                       int* status)
@@ -385,8 +408,10 @@ __global__ void __launch_bounds__(kUT, 2) k_ulv_units(const UlvNode* __restrict_
             const int nt = (n2 + kB - 1) / kB, after = nt - 1 - at / kB;   // blocks; those after this one
             // the diagonal block M (zero outside its triangle, identity past its end) and its
             // inverse, transposed for the second Cholesky sweep
-            const double* const D = Dinv + N.d_off + (MODE == LU_DOWN ? (long long) ((n2 + kB - 1) / kB) * kB * kB : 0) +
+            const long long d_off = N.d_off + (MODE == LU_DOWN ? (long long) ((n2 + kB - 1) / kB) * kB * kB : 0) +
                                     (long long) at * kB;
+            const double* const D = Dinv + d_off;
+            const bool by_subst = subst[d_off / (kB * kB)] != 0;
 #pragma unroll 4
             for (int e = tid; e < kB * kB; e += kUT)
             {
@@ -440,16 +465,24 @@ __global__ void __launch_bounds__(kUT, 2) k_ulv_units(const UlvNode* __restrict_
                 sr[tid] = tid < nr ? b - s : 0.0;
             }
             __syncthreads();
-            // y = M^-1 r, then one step of refinement: y += M^-1 (r - M y)
             const int i = tid >> 2;
-            double y = apply_diag<UP>(sE, sr);
-            if ((tid & 3) == 0) sP[i] = y;
-            __syncthreads();
-            const double d = sr[i] - apply_diag<UP>(sD, sP);
-            if ((tid & 3) == 0) sP[kB + i] = d;
-            __syncthreads();
-            const double c = apply_diag<UP>(sE, sP + kB);
-            if (fabs(c) < HUGE_VAL) y += c;         // not for infinite or NaN unknowns
+            double y;
+            if (by_subst)
+            {
+                if (warp == 0) substitute<UP>(sD, sr, sP);
+                __syncthreads();
+                y = sP[i];
+            } else {
+                // y = M^-1 r, then one step of refinement: y += M^-1 (r - M y)
+                y = apply_diag<UP>(sE, sr);
+                if ((tid & 3) == 0) sP[i] = y;
+                __syncthreads();
+                const double d = sr[i] - apply_diag<UP>(sD, sP);
+                if ((tid & 3) == 0) sP[kB + i] = d;
+                __syncthreads();
+                const double c = apply_diag<UP>(sE, sP + kB);
+                if (fabs(c) < HUGE_VAL) y += c;     // not for infinite or NaN unknowns
+            }
             if ((tid & 3) == 0 && i < nr)
             {
                 const int k = I + at + i;
@@ -534,10 +567,13 @@ __global__ void __launch_bounds__(kUT) k_ulv_form_q(const UlvQJob* __restrict__ 
     }
 }
 
-// Inverse of a diagonal block by substitution, thread c its column c (64 threads).  A block
-// that ends inside the 64 rows is continued with the identity.
+// Inverse E of a diagonal block M by substitution, thread c its column c (64 threads), and the
+// block's flag: the largest row sum of |M| |E| (for Cholesky also of |M^T| |E^T|, which the
+// second sweep solves with) above kInverseMax, or not a number.  A block that ends inside the
+// 64 rows is continued with the identity.
 __global__ void __launch_bounds__(kB) k_ulv_diag(const UlvDiagJob* __restrict__ jobs, const UlvNode* __restrict__ nodes,
-                                                 const double* __restrict__ Lf, double* __restrict__ Dinv)
+                                                 const double* __restrict__ Lf, double* __restrict__ Dinv,
+                                                 unsigned char* __restrict__ subst)
 {
     extern __shared__ __align__(16) double ulv_sm[];
     double* const sD = ulv_sm;                  // the block, row i at sD + i kB
@@ -559,6 +595,28 @@ __global__ void __launch_bounds__(kB) k_ulv_diag(const UlvDiagJob* __restrict__ 
         sx[i * kB + c] = J.unit ? s : s / sD[i * kB + i];
     }
     for (int i = 0; i < kB; i++) Dinv[J.d_off + i * kB + c] = sx[i * kB + c];
+    __shared__ double sum[2][kB];               // row and column sums of |E|
+    __syncthreads();
+    double er = 0.0, ec = 0.0;
+    for (int j = 0; j < kB; j++)
+    {
+        if (J.upper ? j >= c : j <= c) er += fabs(sx[c * kB + j]);
+        if (J.upper ? j <= c : j >= c) ec += fabs(sx[j * kB + c]);
+    }
+    sum[0][c] = er;
+    sum[1][c] = ec;
+    __syncthreads();
+    const double diag = J.unit ? 1.0 : fabs(sD[c * kB + c]);
+    double fr = diag * er, fc = diag * ec;
+    for (int j = 0; j < kB; j++)
+    {
+        if (J.upper ? j > c : j < c) fr = fma(fabs(sD[c * kB + j]), sum[0][j], fr);
+        if (J.upper ? j < c : j > c) fc = fma(fabs(sD[j * kB + c]), sum[1][j], fc);
+    }
+    const bool chol = !J.upper && !J.unit;
+    const double f = chol && !(fc <= fr) ? fc : fr;
+    const int bad = __syncthreads_or(!(f <= kInverseMax));
+    if (c == 0) subst[J.d_off / (kB * kB)] = (unsigned char) (bad != 0);
 }
 
 __global__ void k_ulv_gather(int n, const double* __restrict__ src, const int* __restrict__ map,
@@ -592,6 +650,7 @@ struct h2gpu_ulv {
     Tagged* d_tag = nullptr;             // four tagged vectors: two per sweep
     int* d_ticket = nullptr;             // unit counters, one per level and sweep
     int* h_status = nullptr;             // pinned; set by a wait that ran out
+    unsigned char* d_subst = nullptr;    // per diagonal block: solved by substitution
     double *d_Q = nullptr, *d_L = nullptr, *d_D = nullptr, *d_px = nullptr, *d_b = nullptr, *d_x = nullptr;
     int *d_idx = nullptr, *d_p = nullptr, *d_fwd = nullptr, *d_bwd = nullptr;
     size_t bytes = 0;
@@ -619,7 +678,7 @@ int cuda_status(cudaError_t e, const char* what)
 
 void free_ulv(h2gpu_ulv* u)
 {
-    for (void* p : {(void*) u->d_nodes, (void*) u->d_units, (void*) u->d_tag, (void*) u->d_ticket, (void*) u->d_Q, (void*) u->d_L, (void*) u->d_D, (void*) u->d_px,
+    for (void* p : {(void*) u->d_nodes, (void*) u->d_units, (void*) u->d_tag, (void*) u->d_ticket, (void*) u->d_subst, (void*) u->d_Q, (void*) u->d_L, (void*) u->d_D, (void*) u->d_px,
                     (void*) u->d_b, (void*) u->d_x, (void*) u->d_idx, (void*) u->d_p, (void*) u->d_fwd,
                     (void*) u->d_bwd})
         if (p) cudaFree(p);
@@ -650,8 +709,8 @@ cudaError_t launch_level(h2gpu_ulv* u, int l, cudaStream_t st)
     Tagged* const w = u->d_tag + 2 * down * u->ni;
     // two CTAs per SM (the launch bound); fewer when the level has fewer units
     k_ulv_units<MODE><<<std::min(n, 2 * 148), kUT, smem_bytes(u->q_cap), st>>>(
-        u->d_nodes, u->d_units + b, n, u->d_ticket + down * (u->max_level + 1) + l, u->q_cap, u->d_Q, u->d_L, u->d_D, u->d_idx,
-        u->d_p, u->d_px, w, w + u->ni, u->h_status);
+        u->d_nodes, u->d_units + b, n, u->d_ticket + down * (u->max_level + 1) + l, u->q_cap, u->d_Q, u->d_L, u->d_D, u->d_subst,
+        u->d_idx, u->d_p, u->d_px, w, w + u->ni, u->h_status);
     return cudaGetLastError();
 }
 
@@ -852,7 +911,7 @@ H2G_API int h2gpu_ulv_create(const h2gpu_ulv_desc* d, h2gpu_ulv** out)
         alloc((void**) &u->d_tag, 4 * sizeof(Tagged) * (size_t) ni) &&
         alloc((void**) &u->d_ticket, 2 * sizeof(int) * (size_t) (d->max_level + 1)) &&
         alloc((void**) &u->d_Q, 8 * (size_t) nq) && alloc((void**) &u->d_L, 8 * (size_t) nl) &&
-        alloc((void**) &u->d_D, 8 * (size_t) nd) &&
+        alloc((void**) &u->d_D, 8 * (size_t) nd) && alloc((void**) &u->d_subst, (size_t) nd / (kB * kB)) &&
         alloc((void**) &u->d_idx, 4 * (size_t) ni) && alloc((void**) &u->d_p, 4 * (size_t) np) &&
         alloc((void**) &u->d_fwd, 4 * (size_t) n) && alloc((void**) &u->d_bwd, 4 * (size_t) n) &&
         alloc((void**) &u->d_px, 8 * (size_t) n) && alloc((void**) &u->d_b, 8 * (size_t) n) &&
@@ -880,7 +939,7 @@ H2G_API int h2gpu_ulv_create(const h2gpu_ulv_desc* d, h2gpu_ulv** out)
         step(uploads_landed(), "diagonal blocks") &&
         step(cudaFuncSetAttribute(k_ulv_diag, cudaFuncAttributeMaxDynamicSharedMemorySize, 16 * kB * kB), "diagonal blocks"))
     {
-        k_ulv_diag<<<(unsigned) djobs.size(), kB, 16 * kB * kB, u->stream>>>(d_djobs, u->d_nodes, u->d_L, u->d_D);
+        k_ulv_diag<<<(unsigned) djobs.size(), kB, 16 * kB * kB, u->stream>>>(d_djobs, u->d_nodes, u->d_L, u->d_D, u->d_subst);
         step(cudaGetLastError(), "diagonal blocks");
         step(cudaStreamSynchronize(u->stream), "diagonal blocks");
     }

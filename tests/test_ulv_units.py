@@ -84,3 +84,58 @@ def test_a_solve_right_after_create_sees_whole_factors(lu):
         x = np.empty(n)
         assert u.lib.h2gpu_ulv_solve(u.handle, 3, _dptr(b), _dptr(x)) == 0
         assert np.linalg.norm(x - e) < 1e-13 * np.linalg.norm(e), (n, lu)
+
+
+def _triangle(n, kind, lower, unit):
+    """A triangular factor whose 64 x 64 diagonal blocks M are badly conditioned: "growth": entries -a
+    beside a unit diagonal, || |M| |M^-1| || about (1 + a)^63 (a = 2^17: past the range of a
+    double); "graded": rows scaled from 1 to 1e-14 within every block."""
+    import numpy as np
+    if kind == "graded":
+        T = np.random.default_rng(n).standard_normal((n, n))
+        np.fill_diagonal(T, 1.0)
+        if not unit:
+            T *= 10.0 ** (-14.0 * (np.arange(n) % 64) / 63.0)[:, None]
+    else:
+        T = np.full((n, n), -kind)
+        np.fill_diagonal(T, 1.0)
+    return np.tril(T) if lower else np.triu(T)
+
+
+@pytest.mark.parametrize("lu", [False, True])
+@pytest.mark.parametrize("kind", [0.05, 0.15, 0.3, 1.0, 4.0, 131072.0, "graded"])
+@pytest.mark.parametrize("n", [50, 64, 200])
+def test_ill_conditioned_diagonal_blocks(n, kind, lu):
+    """The residual of a solve is that of substitution, whatever the blocks' conditioning: every
+    row within n units of 1.1e-16 of |T| |x| (Higham, Accuracy and Stability, 8.1), here with
+    a factor of two for the blocks that are solved with their inverse and one refinement (a residual
+    of another 2e-18 of the block's right-hand side).  T x is formed in extended precision.  With
+    a = 2^17 and whole numbers for unknowns substitution is exact, while the inverse overflows."""
+    import numpy as np
+    import torch
+    from perf import cases
+    case = {"kind": "ulv", "n": n, "leaf": n, "frac": 0.5, "frac_up": 0.5, "lu": lu, "op": 1}
+    T0, T1 = _triangle(n, kind, True, lu), _triangle(n, kind, False, False)
+    exact = kind == 131072.0
+
+    def change(u):
+        u.L[0] = torch.from_numpy(np.tril(T0, -1) + T1 if lu else T0).cuda()
+
+    u = _Kept(case, 4, change)
+    u.create()
+    for op in (1, 2):
+        T = T0 if op == 1 else (T1 if lu else T0.T)
+        z = np.random.default_rng(7).integers(1, 9, n).astype(float)
+        r = T @ (z if exact else z + np.random.default_rng(8).random(n))
+        b = np.empty(n)
+        b[u.fwd[u.p[0]] if lu and op == 1 else u.fwd] = r
+        x = torch.empty(n, dtype=torch.float64, device="cuda")
+        cases.run({"kind": "ulv", "ulv": u, "op": op, "b": torch.from_numpy(b).cuda(), "x": x})
+        torch.cuda.synchronize()
+        v = x.cpu().numpy()[u.fwd]
+        if exact:
+            assert np.array_equal(v, z), op
+            continue
+        W = T.astype(np.longdouble)
+        res = np.abs(W @ v - r) / (np.abs(W) @ np.abs(v))
+        assert float(res.max()) < 2 * n * 1.1e-16, (op, float(res.max()))
