@@ -2035,7 +2035,26 @@ int run_panel(h2gpu_image* im, int NV, int nv, const double* X, long long x_rs, 
     // sweep needs too, starts after the upward sweep (Coulomb N = 30,011, 3 right-hand sides:
     // 0.92 one after the other, 0.99 from the fork on, 0.84 so); stored blocks and FP32 gain
     // from the fork on (Coulomb N = 80,000, FP64: 1.01 against 1.05 ms).
-    cudaStream_t c = im->chain;
+    // Inside a caller's capture both run on the caller's stream, the chain first: the image's
+    // chain stream would belong to that capture until the caller ends it, and any other apply
+    // of the image until then (another stream, another capture) would fail and break it.
+    // h2gpu_graph_capture's own capture begins and ends under the image's lock.
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(s, &cap));
+    const bool fork = has_chain(im) && (cap == cudaStreamCaptureStatusNone || s == im->stream);
+    cudaStream_t c = fork ? im->chain : s;
+    // the caller's stream waits for the chain on every return, after a failed launch too
+    struct Join {
+        h2gpu_image* im;
+        cudaStream_t s;
+        bool open;
+        ~Join()
+        {
+            if (!open) return;
+            cudaEventRecord(im->ev_join, im->chain);
+            cudaStreamWaitEvent(s, im->ev_join, 0);
+        }
+    } join{im, s, false};
     if (timed) CK(cudaEventRecord(e[0], s));
     CK(launch_gather(NV, X, x_rs, x_cs, nv, im->d_fwd, im->N, im->d_XS, s));
     if (wide) CK(launch_split3(im->d_XS, 0, im->N, xs_rows, im->d_XS3, s));
@@ -2043,8 +2062,12 @@ int run_panel(h2gpu_image* im, int NV, int nv, const double* X, long long x_rs, 
     if (timed) CK(cudaEventRecord(e[1], s));
     if (has_chain(im))
     {
-        CK(cudaEventRecord(im->ev_fork, s));
-        CK(cudaStreamWaitEvent(c, im->ev_fork, 0));
+        if (fork)
+        {
+            CK(cudaEventRecord(im->ev_fork, s));
+            CK(cudaStreamWaitEvent(c, im->ev_fork, 0));
+            join.open = true;
+        }
         for (size_t L = 0; L + 1 < im->up_beg.size(); L++)
         {
             int b = im->up_beg[L], n = im->up_beg[L + 1] - b;
@@ -2052,7 +2075,7 @@ int run_panel(h2gpu_image* im, int NV, int nv, const double* X, long long x_rs, 
             else CK(launch_up<double>(NV, im->d_up + b, n, im->d_U64, im->d_XS, c));
         }
         if (timed) CK(cudaEventRecord(e[3], c));
-        if (im->BD_JIT && !f32)
+        if (fork && im->BD_JIT && !f32)
         {
             CK(cudaEventRecord(im->ev_join, c));
             CK(cudaStreamWaitEvent(s, im->ev_join, 0));
@@ -2090,7 +2113,7 @@ int run_panel(h2gpu_image* im, int NV, int nv, const double* X, long long x_rs, 
             else CK(launch_down<double>(NV, im->d_dn + b, n, im->d_U64, im->d_Y1, im->d_PS, im->d_PUSH, c));
         }
         if (timed) CK(cudaEventRecord(e[5], c));
-        CK(cudaEventRecord(im->ev_join, c));
+        if (fork) CK(cudaEventRecord(im->ev_join, c));
     }
     // the near field, on the caller's stream
     if (!im->BD_JIT)
@@ -2115,7 +2138,11 @@ int run_panel(h2gpu_image* im, int NV, int nv, const double* X, long long x_rs, 
         im->st.n_launches += panels ? 2 : 0;
     }
     if (timed) CK(cudaEventRecord(e[2], s));
-    if (has_chain(im)) CK(cudaStreamWaitEvent(s, im->ev_join, 0));
+    if (fork)
+    {
+        CK(cudaStreamWaitEvent(s, im->ev_join, 0));
+        join.open = false;
+    }
     if (wide) CK(launch_asm(NV, im->d_asmw, im->n_asmw, im->d_asm_slotsw, im->d_PS, im->d_fwd, Y, y_rs, y_cs, nv, im->N, s));
     else CK(launch_asm(NV, im->d_asm, im->n_asm, im->d_asm_slots, im->d_PS, im->d_fwd, Y, y_rs, y_cs, nv, im->N, s));
     if (timed && uses_status(im, NV))

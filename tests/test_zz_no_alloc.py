@@ -91,3 +91,70 @@ def test_noalloc_refuses_mixed_image_before_its_first_apply():
         assert torch.isfinite(y).all()
     finally:
         img.close()
+
+
+class Captures:
+    """Relaxed captures of torch streams, all ended when the block is left, then replayed."""
+
+    def __enter__(self):
+        from cuda.bindings import runtime as rt
+        self.rt, self.open, self.graphs = rt, [], []
+        return self
+
+    def _do(self, r):
+        assert r[0] == self.rt.cudaError_t.cudaSuccess, r[0]
+        return r[-1]
+
+    def begin(self):
+        import torch
+        s = torch.cuda.Stream()
+        self._do(self.rt.cudaStreamBeginCapture(s.cuda_stream, self.rt.cudaStreamCaptureMode.cudaStreamCaptureModeRelaxed))
+        self.open.append(s)
+        return s
+
+    def __exit__(self, *err):
+        ends = [self.rt.cudaStreamEndCapture(s.cuda_stream) for s in self.open]
+        if err[0] is None:
+            self.graphs = [self._do(r) for r in ends]
+
+    def replay(self):
+        for g, s in zip(self.graphs, self.open):
+            ex = self._do(self.rt.cudaGraphInstantiate(g, 0))
+            self._do(self.rt.cudaGraphLaunch(ex, s.cuda_stream))
+            s.synchronize()
+            self._do(self.rt.cudaGraphExecDestroy(ex))
+            self._do(self.rt.cudaGraphDestroy(g))
+
+
+@pytest.mark.parametrize("kernel,mode,precision", [("coulomb", "jit", "fp64"), ("gaussian", "jit", "mixed"),
+                                                   ("coulomb", "generate", "fp64"), ("coulomb", "generate", "mixed")])
+def test_an_open_capture_leaves_the_image_free(kernel, mode, precision):
+    """The no-allocation apply captured on a caller's stream: until that capture ends, the image
+    takes applies on other streams, host calls and a second capture, and both graphs replay to
+    the eager result."""
+    import torch
+    from perf import cases
+    case = {"kind": "apply", "kernel": kernel, "n": 6000, "leaf": 300, "mode": mode, "precision": precision, "api": "device"}
+    rep = cases.Rep(case, 6000, 9)
+    assert len(rep.adm)
+    img = cases.Image(rep.describe(), precision, blocks="generate" if mode == "generate" else "given")
+    X = cases._rhs(case, 6000, 2, 9)
+    Y, x = img.matmul_device(X), X[:, 0].contiguous()
+    y0 = img.matmul_device(x[:, None])[:, 0].clone()
+    Y2, y1, y2, y3 = torch.empty_like(Y), torch.empty_like(x), torch.empty_like(x), torch.empty_like(x)
+    img.matvec_device_noalloc(x, y3)
+    torch.cuda.synchronize()
+    other = torch.cuda.Stream()
+    xh = x.cpu().numpy()
+    with Captures() as c:
+        img.matvec_device_noalloc(x, y1, stream=c.begin())
+        img.matmul_device(X, Y2, stream=other)
+        img.matvec_device_noalloc(x, y2, stream=c.begin())
+        yh = img.matvec(xh)
+    torch.cuda.synchronize()
+    c.replay()
+    same = 1e-13 if precision == "fp64" else 2e-6
+    assert rel(Y2.cpu(), Y.cpu()) < same and rel(yh, y0.cpu()) < same
+    for y in (y1, y2, y3):
+        assert rel(y.cpu(), y0.cpu()) < same
+    img.close()
