@@ -2150,6 +2150,9 @@ int run_panel(h2gpu_image* im, int NV, int nv, const double* X, long long x_rs, 
     if (timed) CK(cudaEventRecord(e[6], s));
     im->st.n_launches += 4 + (long long) (im->up_beg.size() - 1) + (long long) (im->dn_beg.size() - 1)
                          + (im->BD_JIT ? 0 : 1);
+    if (f32 && !im->BD_JIT && NV == 1)       // lists with warp and CTA tasks: two launches
+        for (int li = 0; li < 2; li++)
+            im->st.n_launches += im->blk1_small[li][1] > 0 && im->blk1_small[li][1] < (li ? im->n_blkD : im->n_blkB);
     return H2GPU_OK;
 }
 

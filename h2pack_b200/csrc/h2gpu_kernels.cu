@@ -381,7 +381,7 @@ __device__ __forceinline__ void chunk_apply(const TA* __restrict__ A, int R, int
         for (int i = threadIdx.x; i < R * NV; i += kThreads) out0[i] = s_o0[i];
 }
 
-// Stored blocks, single right-hand side (the matvec path, memory bound).  One launch.
+// Stored blocks, single right-hand side (the matvec path, memory bound).
 // A task of at most 256 columns, 512 rows and 128 KB (blk1_fits: the B blocks of the
 // usual leaf sizes, and their D blocks in FP32) is one warp's, 8 per CTA; every warp runs
 // its own task, so independent load chains hide each other's latency (one CTA per task
@@ -462,7 +462,7 @@ __device__ __forceinline__ void blk1_warp(const BlkTask& T, const double* __rest
 }
 
 __device__ __forceinline__ void blk1_warp(const BlkTask& T, const float* __restrict__ arena,
-                                          const double* __restrict__ XS, double* __restrict__ PS, double*, int lane)
+                                          const double* __restrict__ XS, double* __restrict__ PS, int lane)
 {
     const int ncol = T.ncol, nrow = T.nrow, ld = T.ld32;
     const bool do0 = T.out0_row >= 0, do1 = T.out1_row >= 0;
@@ -652,11 +652,12 @@ __device__ __forceinline__ void blk1_cta(const BlkTask& T, const TA* __restrict_
 }
 
 
-// CTAs [0, ceil(n_small / 8)): 8 small tasks each, one per warp; the rest: one larger
-// task each (tasks [n_small, n)).
-template <typename TA>
-__global__ void __launch_bounds__(256, sizeof(TA) == 4 ? 2 : 3) k_blk1(const BlkTask* __restrict__ tasks, int n, int n_small,
-                                              const TA* __restrict__ arena, const double* __restrict__ XS,
+// FP64 list: CTAs [0, ceil(n_small / 8)) take 8 small tasks each, one per warp; the rest one
+// larger task each (tasks [n_small, n)).  The two column passes of blk1_warp spill 64 bytes at 80
+// registers; without the spill, at 16 warps an SM and the larger tasks in a launch of their own, the
+// same or slower (Coulomb N = 80,000: 0.90 both, N = 19,000 with 64 leaves: 0.25 -> 0.27 ms).
+__global__ void __launch_bounds__(256, 3) k_blk1(const BlkTask* __restrict__ tasks, int n, int n_small,
+                                              const double* __restrict__ arena, const double* __restrict__ XS,
                                               double* __restrict__ PS)
 {
     __shared__ double s_q[kWarps][256];
@@ -676,8 +677,29 @@ __global__ void __launch_bounds__(256, sizeof(TA) == 4 ? 2 : 3) k_blk1(const Blk
     if (t < n)
     {
         const BlkTask T = tasks[t];
-        blk1_cta<TA>(T, arena, XS, PS, s_q);
+        blk1_cta<double>(T, arena, XS, PS, s_q);
     }
+}
+
+// FP32 list: its small tasks, eight a CTA (both passes' entries in flight take 128 registers), and the
+// larger ones in a launch of their own with the 24 warps an SM that they have registers for.  In
+// one kernel of 128 registers the larger ones had 16: Coulomb N = 160,000, leaves of 312 points:
+// 1.38 -> 1.16 ms a matvec; RPY N = 19,000: 1.17 -> 0.98.
+__global__ void __launch_bounds__(256, 2) k_blk1w(const BlkTask* __restrict__ tasks, int n, const float* __restrict__ arena,
+                                                 const double* __restrict__ XS, double* __restrict__ PS)
+{
+    const int t = blockIdx.x * kWarps + (int) (threadIdx.x >> 5);
+    if (t >= n) return;
+    const BlkTask T = tasks[t];
+    blk1_warp(T, arena, XS, PS, threadIdx.x & 31);
+}
+
+__global__ void __launch_bounds__(256, 3) k_blk1c(const BlkTask* __restrict__ tasks, const float* __restrict__ arena,
+                                                 const double* __restrict__ XS, double* __restrict__ PS)
+{
+    __shared__ double s_q[kWarps][256];
+    const BlkTask T = tasks[blockIdx.x];
+    blk1_cta<float>(T, arena, XS, PS, s_q);
 }
 
 // Stored block chunk for panels of NV >= 4: the R x 32 tile of A staged in shared
@@ -4191,7 +4213,13 @@ cudaError_t launch_blk(int NV, const BlkTask* t, int n, const TA* arena, const d
             k_blk_gemm<TA, NVc><<<n, 256, 0, st>>>(t, arena, XS, PS);
         } else if constexpr (NVc == 1) {
             const int ns = n_small < 0 ? 0 : (n_small > n ? n : n_small);
-            k_blk1<TA><<<(ns + kWarps - 1) / kWarps + (n - ns), 256, 0, st>>>(t, n, ns, arena, XS, PS);
+            const int nw = (ns + kWarps - 1) / kWarps;
+            if constexpr (sizeof(TA) == 8) k_blk1<<<nw + (n - ns), 256, 0, st>>>(t, n, ns, arena, XS, PS);
+            else
+            {
+                if (nw > 0) k_blk1w<<<nw, 256, 0, st>>>(t, ns, arena, XS, PS);
+                if (ns < n) k_blk1c<<<n - ns, 256, 0, st>>>(t + ns, arena, XS, PS);
+            }
         } else {
             constexpr int b = chunk_smem_bytes<NVc>();
             cudaError_t e = allow_smem(k_blk<TA, NVc>, b);

@@ -75,3 +75,23 @@ def test_an_apply_right_after_create_sees_whole_uploads(kernel, n, leaf, mode, p
         a.fill(np.nan if a.dtype == np.float64 else 0)
     assert np.linalg.norm(img.matmul(Xh) - Y) < (1e-13 if precision == "fp64" else 2e-6) * np.linalg.norm(Y)
     img.close()
+
+
+def test_lists_of_warp_and_cta_tasks():
+    """Near blocks of about 181 x 181 FP32 values, on both sides of one warp's 128 KB (blk1_fits): a
+    list with tasks of both kinds, whose two launches cover it (2e-6 as above)."""
+    import numpy as np
+    import torch
+    from perf import cases
+    n = 92672
+    case = {"kind": "apply", "kernel": "coulomb", "n": n, "leaf": 300, "mode": "generate", "precision": "mixed", "api": "device"}
+    rep = cases.Rep(case, n, 5)
+    npt = (rep.t["end"] - rep.t["start"])[rep.t["n_child"] == 0]
+    assert 4 * int(npt.min()) ** 2 <= 128 * 1024 < 4 * int(npt.max()) ** 2
+    img = cases.Image(rep.describe(), "mixed", blocks="generate")
+    x = cases._rhs(case, n, 1, 5)
+    y, e = img.matmul_device(x), rep.apply(x)
+    torch.cuda.synchronize()
+    assert float((y - e).norm() / e.norm()) < 2e-6
+    assert np.linalg.norm(img.matvec(x[:, 0].cpu().numpy()) - e[:, 0].cpu().numpy()) < 2e-6 * float(e.norm())
+    img.close()
