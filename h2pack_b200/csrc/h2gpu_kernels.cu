@@ -1361,7 +1361,7 @@ __device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b)
     asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};" : "+d"(d[0]), "+d"(d[1]) : "d"(a), "d"(b));
 }
 
-// A chunk of <= 128 target points and a share of its source tiles per CTA, four CTAs per SM.
+// A chunk of <= 128 target points and a share of its source tiles per CTA (Jit64Cfg::CTAS per SM).
 // What bounds it: the FP64 pipe (a kernel value takes 14 to 25 operations, each right-hand
 // side one more, in DMMA as in DFMA: 17 and 18 T multiply-adds/s measured, not in
 // addition).  A warp walks 32 targets, four sources at a time: a lane evaluates source
@@ -1376,9 +1376,9 @@ __device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b)
 // a DMMA's A fragment; others: multiply-adds into the lane's own sums, added over lane % 4
 // at the end.  Warps that a chunk leaves over (<= 64 or <= 32 targets) take every 2nd or
 // 4th step of the sources.  Small images have fewer chunks than the GPU has CTA slots:
-// there the CTAs of a cluster share a chunk, each taking every S-th source tile, and their
-// sums meet in the first CTA through distributed shared memory, in rank order.  Outputs are
-// written once, no atomics.
+// there the CTAs of a cluster share a chunk, each taking every S-th source tile; then each adds,
+// in rank order, all the CTAs' sums of its part of the outputs through distributed shared
+// memory.  Outputs are written once, no atomics.
 template <int NV, int KD> struct Jit64Cfg {
     static constexpr int W = KD * NV;
     static constexpr bool MMA = KD == 1 && NV >= 8;
@@ -1391,6 +1391,11 @@ template <int NV, int KD> struct Jit64Cfg {
     // warps per SM: 16 of 128 registers; four RPY values at once take 168 (3.5 -> 0.98 ms for N =
     // 20,011, one right-hand side; 1.03 ms with 128 and spills)
     static constexpr int CTAS = (KD == 3 && G == 4 ? 384 : 512) / NT;
+    // CTAs per SM that jit_split counts.  RPY with one or two right-hand sides fits 3 and 2, but is
+    // split as for 4: with the true counts N = 10,000, leaves of 100, took 508 instead of 473 us
+    // (1) and 627 instead of 611 (2) at 2.3 waves, N = 20,011 988 instead of 1,059 (2).  Wider
+    // panels: counted as 4, N = 6,000 took 583 instead of 454 us (4) and 1,185 instead of 950 (8).
+    static constexpr int SLOTS = CTAS == 1 ? 1 : 4;
 };
 template <int KID, int NV, int KD>
 __global__ void __launch_bounds__(Jit64Cfg<NV, KD>::NT, Jit64Cfg<NV, KD>::CTAS)
@@ -4393,14 +4398,13 @@ static cudaError_t launch_jit_k(int NV, const JitTarget* tg, int n, const void* 
         }
     }
     // FP32: two targets per thread (64 threads per 128-point chunk) where the accumulators
-    // allow it; FP64: one target per thread (two took 188 registers and left 7 warps per SM
-    // to hide the FP64 latencies: 1.4x slower)
+    // allow it; FP64: Jit64Cfg's targets per lane
     NV_DISPATCH(NV, {
         if constexpr (KD == 3 && NVc > 8)
             return cudaErrorInvalidValue;   // tensor kernels run in panels of <= 8 right-hand sides
         else if constexpr (sizeof(T) == 8)
         {
-            const JitSplit sp = jit_split(n, 4, 2);
+            const JitSplit sp = jit_split(n, Jit64Cfg<NVc, KD>::SLOTS, 2);
             return launch_cluster(k_jit64<KID, NVc, KD>, n * sp.parts, sp.share, Jit64Cfg<NVc, KD>::NT, 0, st, tg, tiles, p,
                                   kp, XS, PS, Y1, sp.parts, sp.share);
         }
@@ -4408,7 +4412,7 @@ static cudaError_t launch_jit_k(int NV, const JitTarget* tg, int n, const void* 
         {
             // scalar FP32 kernels: the two targets of a thread as one FP32x2 pair
             if (!use_shift) return cudaErrorInvalidValue;   // FP32 evaluation is re-centred
-            const int S = jit_split(n, 8, 1).share;
+            const int S = jit_split(n, NVc >= 16 ? 8 : 10, 1).share;   // its CTAs per SM
             return launch_cluster(far ? k_jit2<KID, NVc, true> : k_jit2<KID, NVc, false>, n, S, 64, 0, st, tg, tiles,
                                   (const float4*) pts, kp, XS, PS, Y1, lo, S);
         }
