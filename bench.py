@@ -289,32 +289,39 @@ def run_ours(args):
                 e.append(float(np.linalg.norm(Yc[rows, c] - yd) / np.linalg.norm(yd)))
             err[name] = max(e)
 
-    # ---- roofline of the dominant kernel (far-field JIT: on-the-fly B blocks x 16 RHS)
+    # ---- roofline of the dominant kernel (k_jit_tc: on-the-fly B and D blocks x 16 RHS).  The two
+    # fields run beside each other, and each phase's time holds half of what it shares: the
+    # operations of both over the time of both (the sweeps' share of the overlap included)
     st = img.stats()
-    flop_per_pair = 13 + 4 * nv      # Matern32_3D_krnl_bimv_flop = 17 per pair for one RHS, 4 of them the bi-matvec
-    far_flops = st["jit_pairs_B"] * flop_per_pair
-    far_ms = phase[1]
+    d = H.describe()
+    diag = sum(float(d.pt_cluster[2 * i + 1] - d.pt_cluster[2 * i] + 1) ** 2 for i in d.leaf_nodes[:d.n_leaf_node])
+    pairs = st["jit_pairs_B"] + st["jit_pairs_D"] - diag
+    # Matern32_3D_krnl_bimv_flop = 17 per unordered pair for one RHS, 4 of them the bi-matvec; the
+    # diagonal blocks take half of that per ordered pair
+    flops = pairs * (13 + 4 * nv) + diag * (13 + 2 * nv)
+    jit_ms = phase[1] + phase[3]
     peaks = measured_peaks(local)
     peak_fp32 = peaks["fp32_tflops"]
-    # MUFU: a Matern-3/2 value costs one rsqrt and one ex2; both directions of an unordered
-    # far-field pair are evaluated (owner computes)
-    mufu_rate = st["jit_pairs_B"] * 4 / (far_ms * 1e-3) / 1e12
+    # MUFU: a Matern-3/2 value costs one sqrt and one ex2; both directions of an unordered
+    # pair are evaluated (owner computes)
+    mufu_rate = (4 * pairs + 2 * diag) / (jit_ms * 1e-3) / 1e12
     # DRAM traffic of one far-field launch from an ncu capture of the N = 125,000 case of
     # this workload (dram__bytes_read.sum + dram__bytes_write.sum = 28.1 MB: source panels,
     # tile records, coordinates, outputs), scaled by N (the traffic is proportional to the
-    # points, not the pairs).  The B phase also holds the skeleton panel fill (< 1 %).
+    # points, not the pairs)
     traffic = (27.70e6 + 0.38e6) * args.n / 125_000
-    roofline = {"bound": "fp32", "kernel": "k_jit_tc (far field, on-the-fly B x 16 RHS, tensor cores; B phase incl. panel fill)",
-                "achieved": far_flops / (far_ms * 1e-3) / 1e12, "peak": peak_fp32, "unit": "TFLOP/s",
-                "frac": far_flops / (far_ms * 1e-3) / 1e12 / peak_fp32, "traffic": traffic,
+    tflops = flops / (jit_ms * 1e-3) / 1e12
+    roofline = {"bound": "fp32", "kernel": "k_jit_tc (far and near field, on-the-fly blocks x 16 RHS, tensor cores; B and D phases)",
+                "achieved": tflops, "peak": peak_fp32, "unit": "TFLOP/s", "frac": tflops / peak_fp32, "traffic": traffic,
                 "traffic_source": "ncu capture of the N=125000 far-field launch, scaled by N",
                 "peak_source": "measured on this GPU by h2gpu_measure_peaks (packed FP32x2 FMA chains on every SM); "
                                f"nominal 148 SM x 128 lanes x 2 x 1.965 GHz = 74.4 TFLOP/s, frac of nominal "
-                               f"{far_flops / (far_ms * 1e-3) / 1e12 / 74.4:.3f}",
-                "flop_model": f"unordered point pairs x ({flop_per_pair}) = H2Pack JIT_flops model with 16 RHS",
+                               f"{tflops / 74.4:.3f}",
+                "flop_model": f"unordered point pairs x ({13 + 4 * nv}), within leaves x ({13 + 2 * nv}) = H2Pack JIT_flops "
+                              "model with 16 RHS",
                 "mufu": {"achieved": mufu_rate, "peak": peaks["mufu_tops"], "unit": "10^12 ops/s",
                          "frac": mufu_rate / peaks["mufu_tops"],
-                         "model": "4 MUFU ops (rsqrt, ex2 per value, both directions) per unordered far-field pair; "
+                         "model": "2 MUFU ops (sqrt, ex2) per value, both directions of an unordered pair; "
                                   "peak measured by h2gpu_measure_peaks (ex2.approx chains)"}}
 
     cpu, parity = None, None

@@ -2079,7 +2079,6 @@ int run_panel(h2gpu_image* im, int NV, int nv, const double* X, long long x_rs, 
         {
             CK(cudaEventRecord(im->ev_join, c));
             CK(cudaStreamWaitEvent(s, im->ev_join, 0));
-            if (timed) CK(cudaEventRecord(e[1], s));
         }
         if (!im->BD_JIT)
         {
@@ -2269,29 +2268,36 @@ int apply_device(h2gpu_image* im, int n_vec, const double* X, long long x_rs, lo
         if (down && c0 + NV >= n_vec) CK(cudaMemcpyAsync(down, Y, down_bytes, cudaMemcpyDeviceToHost, s));
         CK(cudaEventSynchronize(im->ev.e[6]));
         TRY(check_status(im));
-        // the pair plan runs D (1 -> 2) before the chain (2 -> 3 -> 4 -> 5), otherwise both
-        // start after the gather (1) and the assembly follows the later one
-        cudaEvent_t* ev = im->ev.e;
-        const bool pair = pair_plan(im, NV);
-        auto ms = [&](int a, int b) {
-            float t = 0.f;
-            cudaEventElapsedTime(&t, ev[a], ev[b]);
-            return t;
-        };
-        const bool after_up = im->BD_JIT && im->precision == H2GPU_PREC_FP64;   // D's start: run_panel
-        const bool chain = pair || has_chain(im);
-        ph[3] += ms(1, 2);                         // D
-        if (chain)
+        float t[7];                                // end of each step, from the apply's start
+        for (int k = 1; k < 7; k++)
+            if (k < 3 || k > 5 || pair_plan(im, NV) || has_chain(im)) CK(cudaEventElapsedTime(&t[k], im->ev.e[0], im->ev.e[k]));
+        if (pair_plan(im, NV))
         {
-            ph[0] += pair ? ms(0, 1) + ms(2, 3) : after_up ? ms(0, 3) : ms(0, 1) + ms(1, 3);   // gather + upward
-            ph[1] += ms(3, 4);                     // B
-            ph[2] += ms(4, 5);                     // downward
-            ph[4] += std::min(ms(5, 6), ms(2, 6)); // assemble
+            // one step after the other: gather, D, upward, B, downward, assemble
+            const float d[5] = {t[1] + (t[3] - t[2]), t[4] - t[3], t[5] - t[4], t[2] - t[1], t[6] - t[5]};
+            for (int k = 0; k < 5; k++) ph[k] += d[k];
+        } else if (!has_chain(im)) {
+            ph[0] += t[1];
+            ph[3] += t[2] - t[1];
+            ph[4] += t[6] - t[2];
         } else {
-            ph[0] += ms(0, 1);
-            ph[4] += ms(2, 6);
+            // D runs beside the chain, from the fork or the end of the upward sweep on (run_panel):
+            // half of the time that two phases share counts to each, so that the phases add
+            // up to the whole apply
+            const float d0 = im->BD_JIT && im->precision == H2GPU_PREC_FP64 ? t[3] : t[1];
+            const float from[3] = {d0, t[3], t[4]}, to[3] = {t[3], t[4], t[5]};
+            float D = t[2] - d0;
+            ph[0] += d0;
+            for (int k = 0; k < 3; k++)
+            {
+                const float shared = std::max(0.f, std::min(to[k], t[2]) - std::max(from[k], d0));
+                ph[k] += to[k] - from[k] - 0.5f * shared;
+                D -= 0.5f * shared;
+            }
+            ph[3] += D;
+            ph[4] += t[6] - std::max(t[5], t[2]);
         }
-        total += ms(0, 6);
+        total += t[6];
     }
     for (int k = 0; k < 5; k++) im->st.ms_phase[k] += ph[k];
     im->st.ms_total += total;

@@ -160,8 +160,9 @@ typedef struct h2gpu_stats
 {
     long long n_matvec;       /* right-hand sides applied (src/H2Pack_matvec.c:1283)  */
     double ms_total;          /* device time of all applies                           */
-    double ms_phase[5];       /* gather/up, B, down, D, assemble (device events; D runs
-                                 beside the others, so they add up to more than ms_total) */
+    double ms_phase[5];       /* gather/up, B, down, D, assemble (device events); where D runs
+                                 beside another, half of the shared time counts to each:
+                                 they add up to ms_total                               */
     double bytes_U;           /* U bytes read by one upward + one downward sweep       */
     double bytes_B;           /* stored B bytes (AOT)                                  */
     double bytes_D;           /* stored D bytes (AOT)                                  */

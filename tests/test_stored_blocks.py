@@ -95,3 +95,27 @@ def test_lists_of_warp_and_cta_tasks():
     assert float((y - e).norm() / e.norm()) < 2e-6
     assert np.linalg.norm(img.matvec(x[:, 0].cpu().numpy()) - e[:, 0].cpu().numpy()) < 2e-6 * float(e.norm())
     img.close()
+
+
+@pytest.mark.parametrize("kernel,n,mode,precision,variant", [
+    ("coulomb", 6000, "generate", "fp64", None), ("coulomb", 6000, "generate", "mixed", None), ("coulomb", 200, "generate", "mixed", None),
+    ("gaussian", 20000, "jit", "fp64", None), ("gaussian", 20000, "jit", "mixed", "tc"), ("gaussian", 20000, "jit", "mixed", "pair")])
+def test_phase_times_add_up(kernel, n, mode, precision, variant):
+    """h2gpu_get_stats: the phases of any number of applies add up to their device time, with the
+    near field beside the others, one after the other (pair), and without admissible pairs."""
+    from perf import cases
+    case = {"kind": "apply", "kernel": kernel, "n": n, "leaf": 300, "mode": mode, "precision": precision, "api": "device"}
+    rep = cases.Rep(case, n, 4)
+    img = cases.Image(rep.describe(), precision, blocks="generate" if mode == "generate" else "given")
+    if variant:
+        img.set_jit_variant(variant)
+    for nv in (1, 16, 64):
+        X = cases._rhs(case, n, nv, 4)
+        img.matmul_device(X)
+        img.reset_stats()
+        for _ in range(3):
+            img.matmul_device(X)
+        st = img.stats()
+        assert st["ms_total"] > 0 and min(st["ms_phase"]) >= 0
+        assert abs(sum(st["ms_phase"]) - st["ms_total"]) < 1e-4 * st["ms_total"], (nv, st["ms_phase"], st["ms_total"])
+    img.close()
