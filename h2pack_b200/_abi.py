@@ -129,6 +129,7 @@ H2GPU_SYMBOLS = {
     "h2gpu_ulv_destroy": (C.c_int, [C.c_void_p]),
     "h2gpu_ulv_solve": (C.c_int, [C.c_void_p, C.c_int, _dp, _dp]),
     "h2gpu_ulv_solve_device": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p]),
+    "h2gpu_ulv_wait_check": (C.c_int, [C.c_void_p]),
     "h2gpu_ulv_bytes": (C.c_size_t, [C.c_void_p]),
 }
 

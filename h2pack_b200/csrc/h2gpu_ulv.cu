@@ -47,7 +47,8 @@ constexpr int kDS = kB + 4;                // column stride of a diagonal block 
                                            // conflict-free)
 constexpr int kMaxNodeRows = 13872;        // larger nodes are refused
 constexpr unsigned kFull = 0xffffffffu;
-constexpr int kPollLimit = 1 << 22;        // polls (a few seconds) before a wait gives up
+constexpr int kPollLimit = 1 << 22;        // polls (a few seconds) before a wait gives up; looked at
+                                           // every 2^16 polls
 // Largest || |M| |M^-1| || of a diagonal block M that is solved with its inverse E.  One step of
 // refinement leaves a residual of about (128 u || |M| |E| ||)^2 of the block's right-hand
 // side beside the rounding that substitution has too (u = 2^-53): 2e-18 at this bound.
@@ -119,11 +120,11 @@ __device__ __forceinline__ Tagged tag_get(const Tagged* p)
 }
 // the value of an entry whose first read gave r; a wait that runs out sets the status word
 // and returns zero, and every later wait then gives up soon
-__device__ __forceinline__ double tag_wait(const Tagged* p, Tagged r, int* status)
+__device__ __forceinline__ double tag_wait(const Tagged* p, Tagged r, int* status, int limit)
 {
     for (int n = 1; r.t == 0; n++)
     {
-        if ((n & 0xffff) == 0 && (n >= kPollLimit || *(volatile int*) status != 0))
+        if ((n & 0xffff) == 0 && (n >= limit || *(volatile int*) status != 0))
         {
             *(volatile int*) status = 1;
             return 0.0;
@@ -138,9 +139,10 @@ __device__ __forceinline__ double tag_wait(const Tagged* p, Tagged r, int* statu
 struct InTagged {
     const Tagged* x;
     int* status;
+    int limit;
     using R = Tagged;
     __device__ R issue(int c) const { return tag_get(x + c); }
-    __device__ double wait(int c, R r) const { return tag_wait(x + c, r, status); }
+    __device__ double wait(int c, R r) const { return tag_wait(x + c, r, status, limit); }
     // entries c0 and c1 (those below n) together: one round trip where both are new
     __device__ void wait2(int c0, int c1, int n, R r0, R r1, double& v0, double& v1) const
     {
@@ -148,7 +150,7 @@ struct InTagged {
         const bool two = c1 < n;
         for (int k = 1; r0.t == 0 || (two && r1.t == 0); k++)
         {
-            if ((k & 0xffff) == 0 && (k >= kPollLimit || *(volatile int*) status != 0))
+            if ((k & 0xffff) == 0 && (k >= limit || *(volatile int*) status != 0))
             {
                 *(volatile int*) status = 1;
                 return;
@@ -363,7 +365,7 @@ __global__ void __launch_bounds__(kUT, 2) k_ulv_units(const UlvNode* __restrict_
                                                       const unsigned char* __restrict__ subst,
                                                       const int* __restrict__ idxs, const int* __restrict__ piv,
                                                       double* px, Tagged* W, Tagged* X,
-                                                      int* status)
+                                                      int* status, int limit)
 {
     constexpr bool UP = MODE == CH_UP || MODE == LU_UP;
     extern __shared__ __align__(16) double ulv_sm[];
@@ -431,12 +433,12 @@ __global__ void __launch_bounds__(kUT, 2) k_ulv_units(const UlvNode* __restrict_
                 if constexpr (UP)
                 {
                     const int k = I + (MODE == LU_UP ? piv[N.p_off + i] : i);
-                    b = hasq ? tag_wait(w + k, tag_get(w + k), status) : px[idx[k]];
+                    b = hasq ? tag_wait(w + k, tag_get(w + k), status, limit) : px[idx[k]];
                 } else b = px[idx[I + i]];
             }
             double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
             double2 ac = make_double2(0.0, 0.0);
-            const InTagged xs{x + I, status};
+            const InTagged xs{x + I, status, limit};
             if constexpr (UP)
                 rows_product(T + (long long) at * m, m, nr, n2, 0, 1, at / kB, xs, acc);
             else if constexpr (MODE == LU_DOWN)
@@ -494,9 +496,9 @@ __global__ void __launch_bounds__(kUT, 2) k_ulv_units(const UlvNode* __restrict_
         {
             const int nr = min(kB, I - at);
             double b = 0.0;
-            if (tid < nr) b = hasq ? tag_wait(w + at + tid, tag_get(w + at + tid), status) : px[idx[at + tid]];
+            if (tid < nr) b = hasq ? tag_wait(w + at + tid, tag_get(w + at + tid), status, limit) : px[idx[at + tid]];
             double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-            rows_product(L + (long long) at * m + I, m, nr, n2, 0, 1, (n2 + kB - 1) / kB, InTagged{x + I, status}, acc);
+            rows_product(L + (long long) at * m + I, m, nr, n2, 0, 1, (n2 + kB - 1) / kB, InTagged{x + I, status, limit}, acc);
             rows_reduce(acc, sP);
             __syncthreads();
             if (tid < nr)
@@ -508,7 +510,7 @@ __global__ void __launch_bounds__(kUT, 2) k_ulv_units(const UlvNode* __restrict_
         }
         else if (un.type == U_Q)
         {
-            for (int i = tid; i < m; i += kUT) sx[i] = i < I ? px[idx[i]] : tag_wait(x + i, tag_get(x + i), status);
+            for (int i = tid; i < m; i += kUT) sx[i] = i < I ? px[idx[i]] : tag_wait(x + i, tag_get(x + i), status, limit);
             __syncthreads();
             const int nc = min(kB, m - at);
             double2 ac = make_double2(0.0, 0.0);
@@ -528,7 +530,7 @@ __global__ void __launch_bounds__(kUT, 2) k_ulv_units(const UlvNode* __restrict_
         {
             // U_PUT: the first sweep's results are in x (b1 and b2), the second's in w
             const Tagged* const r = UP ? x : w;
-            for (int i = tid; i < m; i += kUT) tag_wait(r + i, tag_get(r + i), status);
+            for (int i = tid; i < m; i += kUT) tag_wait(r + i, tag_get(r + i), status, limit);
             __syncthreads();
             for (int i = tid; i < m; i += kUT) px[idx[i]] = __longlong_as_double(tag_get(r + i).v);
         }
@@ -700,17 +702,18 @@ struct DeviceGuard {
     }
 };
 
+// skip, limit: the level's first units left out, and the polls of a wait (h2gpu_ulv_wait_check)
 template <int MODE>
-cudaError_t launch_level(h2gpu_ulv* u, int l, cudaStream_t st)
+cudaError_t launch_level(h2gpu_ulv* u, int l, cudaStream_t st, int skip = 0, int limit = kPollLimit)
 {
     constexpr int down = MODE == CH_DOWN || MODE == LU_DOWN;
-    const int b = u->beg[down][l], n = u->beg[down][l + 1] - b;
+    const int b = u->beg[down][l] + skip, n = u->beg[down][l + 1] - b;
     if (n <= 0) return cudaSuccess;
     Tagged* const w = u->d_tag + 2 * down * u->ni;
     // two CTAs per SM (the launch bound); fewer when the level has fewer units
     k_ulv_units<MODE><<<std::min(n, 2 * 148), kUT, smem_bytes(u->q_cap), st>>>(
         u->d_nodes, u->d_units + b, n, u->d_ticket + down * (u->max_level + 1) + l, u->q_cap, u->d_Q, u->d_L, u->d_D, u->d_subst,
-        u->d_idx, u->d_p, u->d_px, w, w + u->ni, u->h_status);
+        u->d_idx, u->d_p, u->d_px, w, w + u->ni, u->h_status, limit);
     return cudaGetLastError();
 }
 
@@ -722,14 +725,19 @@ int check_waits(h2gpu_ulv* u)
     return ulv_fail(H2GPU_ERR_DEVICE, "ULV solve: a bounded wait between units expired");
 }
 
+cudaError_t start_solve(h2gpu_ulv* u, const double* d_b, cudaStream_t st)
+{
+    const int gs = (int) std::max<long long>(1, std::min<long long>((std::max<long long>(u->n, 4 * u->ni) + 255) / 256, 148 * 8));
+    k_ulv_start<<<gs, 256, 0, st>>>(u->n, d_b, u->d_fwd, u->d_px, u->d_tag, 4 * u->ni, u->d_ticket, 2 * (u->max_level + 1));
+    return cudaGetLastError();
+}
+
 int enqueue_solve(h2gpu_ulv* u, int op, const double* d_b, double* d_x, cudaStream_t st)
 {
     const int st0 = check_waits(u);
     if (st0 != H2GPU_OK) return st0;
     const int gb = std::max(1, std::min((u->n + 255) / 256, 4096));
-    const int gs = (int) std::max<long long>(1, std::min<long long>((std::max<long long>(u->n, 4 * u->ni) + 255) / 256, 148 * 8));
-    k_ulv_start<<<gs, 256, 0, st>>>(u->n, d_b, u->d_fwd, u->d_px, u->d_tag, 4 * u->ni, u->d_ticket, 2 * (u->max_level + 1));
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = start_solve(u, d_b, st);
     if (op & 1)
         for (int l = u->max_level; l >= 0 && e == cudaSuccess; l--)
             e = u->lu ? launch_level<LU_UP>(u, l, st) : launch_level<CH_UP>(u, l, st);
@@ -1015,6 +1023,24 @@ H2G_API int h2gpu_ulv_solve(h2gpu_ulv* u, int op, const double* b, double* x)
     if (st == H2GPU_OK) st = cuda_status(cudaMemcpyAsync(x, u->d_x, nb, cudaMemcpyDeviceToHost, u->stream), "download");
     const int s2 = cuda_status(cudaStreamSynchronize(u->stream), "solve");
     if (st == H2GPU_OK) st = s2;
+    return st != H2GPU_OK ? st : check_waits(u);
+}
+
+H2G_API int h2gpu_ulv_wait_check(h2gpu_ulv* u)
+{
+    if (!u) return ulv_fail(H2GPU_ERR_INVALID, "ULV wait check: NULL argument");
+    DeviceGuard guard(u->device);
+    const int st0 = check_waits(u);
+    if (st0 != H2GPU_OK) return st0;
+    cudaError_t e = start_solve(u, u->d_x, u->stream);      // the values do not matter
+    for (int l = u->max_level; l >= 0 && e == cudaSuccess; l--)
+        if (u->beg[0][l + 1] - u->beg[0][l] > 1)
+        {
+            e = u->lu ? launch_level<LU_UP>(u, l, u->stream, 1, 1) : launch_level<CH_UP>(u, l, u->stream, 1, 1);
+            break;
+        }
+    const cudaError_t es = cudaStreamSynchronize(u->stream);
+    const int st = cuda_status(e != cudaSuccess ? e : es, "wait check");
     return st != H2GPU_OK ? st : check_waits(u);
 }
 

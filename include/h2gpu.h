@@ -458,6 +458,11 @@ int h2gpu_ulv_solve(h2gpu_ulv *u, int op, const double *b, double *x);
    must not overlap on the device (enqueue them on one stream; the drop-in serialises
    per handle); different objects are independent. */
 int h2gpu_ulv_solve_device(h2gpu_ulv *u, int op, const double *d_b, double *d_x, void *stream);
+/* Self-check of the bounded waits: the first sweep of the deepest level with more than one
+   unit runs without its first unit and with the shortest limit, so that waits run out.
+   Returns H2GPU_ERR_DEVICE, as a solve would; H2GPU_OK if no level has two units.  The next
+   solve is not affected.  Not beside a solve of the same object. */
+int h2gpu_ulv_wait_check(h2gpu_ulv *u);
 size_t h2gpu_ulv_bytes(const h2gpu_ulv *u);
 
 #ifdef __cplusplus

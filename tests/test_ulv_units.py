@@ -139,3 +139,27 @@ def test_ill_conditioned_diagonal_blocks(n, kind, lu):
         W = T.astype(np.longdouble)
         res = np.abs(W @ v - r) / (np.abs(W) @ np.abs(v))
         assert float(res.max()) < 2 * n * 1.1e-16, (op, float(res.max()))
+
+
+@pytest.mark.parametrize("lu", [False, True])
+@pytest.mark.parametrize("n,leaf", [(40, 64), (700, 700), (2001, 40)])
+def test_a_wait_that_runs_out_is_reported_once(n, leaf, lu):
+    """One unit left out, so that the units which read its entries give up at the shortest limit: the
+    check returns H2GPU_ERR_DEVICE, and the next solve is right (one unit alone waits for
+    nothing)."""
+    import torch
+    from h2pack_b200 import _abi
+    from perf import cases
+    case = {"kind": "ulv", "n": n, "leaf": leaf, "frac": 0.6, "frac_up": 0.5, "lu": lu, "op": 3}
+    s = cases.prepare(case, 3)
+    u = s["ulv"]
+    alone = n == 40 and not lu                  # LU: the unit that scatters waits for the block
+    assert u.lib.h2gpu_ulv_wait_check(u.handle) == (_abi.H2GPU_OK if alone else -6)
+    if not alone:
+        assert b"bounded wait" in u.lib.h2gpu_last_error()
+    x = cases.run(s).clone()
+    torch.cuda.synchronize()
+    e = cases.exact(case, 3)
+    assert float((x - e).norm() / e.norm()) < 1e-13
+    assert u.lib.h2gpu_ulv_solve(u.handle, 3, *[a.ctypes.data_as(cases.C.POINTER(cases.C.c_double))
+                                                 for a in (s["b"].cpu().numpy(), x.cpu().numpy())]) == 0
