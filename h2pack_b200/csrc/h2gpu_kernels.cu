@@ -1254,7 +1254,8 @@ __global__ void __launch_bounds__(128 / TPT, 5 * TPT) k_jit(const JitTarget* __r
 // ---------------------------------------------------------- JIT owner kernel, FP64
 //
 // FP64 kernel evaluation.  The FP64 pipe bounds the FP64 path, so the values are formed with
-// as few FP64 operations as a result within about one unit in the last place takes; every
+// as few FP64 operations as a result within about one unit in the last place takes (exp64 1.09
+// by analysis, rsqrt64 0.94, sqrt64 0.50; tested entry by entry over their ranges); every
 // argument outside the fast path's range (zero or denormal or non-finite r^2, |t| >= 700)
 // goes to the CUDA math functions of Scalar<KID, double>.
 

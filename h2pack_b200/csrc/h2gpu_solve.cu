@@ -6,8 +6,9 @@
 // examples/SPDHSS-H2/pcg_tests.c:13-20, run for up to 16 right-hand sides ("slots")
 // at once: the slots are the columns of one 16-wide panel, so every iteration is one
 // H2 matmul (of the panel's columns up to the highest busy slot) plus three small
-// kernels (direction update, p'Ap, alpha, x/r update with ||r||^2, status).  The host only enqueues iterations and reads the
-// 16 slot records once per batch of iterations; it never waits per iteration.
+// kernels: the direction update; p'Ap, whose last block takes alpha; the x / r update with
+// ||r||^2, whose last block takes the slots' status.  The host only enqueues iterations and
+// reads the 16 slot records once per batch of iterations; it never waits per iteration.
 //
 // Precision: vectors, inner products and the residual recomputation are FP64; the
 // operator runs in the image's precision.  A slot whose recursive residual claims

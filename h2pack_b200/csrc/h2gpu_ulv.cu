@@ -45,7 +45,8 @@ constexpr int kUT = 256, kUW = kUT / 32;   // threads and warps of a CTA
 constexpr int kB = 64;                     // rows / columns of a unit
 constexpr int kDS = kB + 4;                // column stride of a diagonal block in shared memory (apply_diag:
                                            // conflict-free)
-constexpr int kMaxNodeRows = 13872;        // larger nodes are refused
+constexpr int kMaxNodeRows = 13872;        // larger nodes are refused: the interface's limit (a Q
+                                           // product would hold some 19,700 in shared memory)
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kPollLimit = 1 << 22;        // polls (a few seconds) before a wait gives up; looked at
                                            // every 2^16 polls
@@ -861,7 +862,7 @@ H2G_API int h2gpu_ulv_create(const h2gpu_ulv_desc* d, h2gpu_ulv** out)
     for (int i = 0; i < d->n_node; i++)
         if (level_of[i] < 0) { nodes[i] = UlvNode{}; nodes[i].q_off = nodes[i].p_off = -1; }
     if (m_cap > kMaxNodeRows)
-        return ulv_fail(H2GPU_ERR_UNSUPPORTED, "a node of %d rows exceeds one CTA's shared memory", m_cap);
+        return ulv_fail(H2GPU_ERR_UNSUPPORTED, "a node of %d rows, more than %d", m_cap, kMaxNodeRows);
     int dev = d->device;
     if (dev < 0 && cudaGetDevice(&dev) != cudaSuccess) return ulv_fail(H2GPU_ERR_CUDA, "no CUDA device");
     DeviceGuard guard(dev);
@@ -980,7 +981,7 @@ H2G_API int h2gpu_ulv_create(const h2gpu_ulv_desc* d, h2gpu_ulv** out)
         int optin = 0;
         if (step(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "device query") &&
             smem_bytes(u->q_cap) > (optin -= 128))      // the kernels' static part is within 128 bytes
-            st = ulv_fail(H2GPU_ERR_UNSUPPORTED, "a node of %d rows exceeds one CTA's shared memory", m_cap);
+            st = ulv_fail(H2GPU_ERR_UNSUPPORTED, "a node of %d rows with a Q exceeds one CTA's shared memory", u->q_cap);
         for (auto kern : {k_ulv_units<CH_UP>, k_ulv_units<CH_DOWN>, k_ulv_units<LU_UP>, k_ulv_units<LU_DOWN>})
             if (st == H2GPU_OK)
                 step(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, optin),

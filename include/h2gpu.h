@@ -260,8 +260,10 @@ int h2gpu_autotune(h2gpu_image *img, int n_vec, const double *dX, int ldx, doubl
  * H2GPU_JIT_TC (default: block products of panels of 8 or 16 on the tensor cores with
  * warp-level MMAs, 3xTF32), H2GPU_BLK_TCGEN05 (the same on tcgen05: values split into
  * three BF16 pieces, six products kept, accumulators in tensor memory) or
- * H2GPU_JIT_SIMT (CUDA cores).  FP64 panels always use the CUDA cores; a captured
- * graph keeps the variant it was captured with.  No counterpart in the reference.
+ * H2GPU_JIT_SIMT (CUDA cores).  FP64 panels have one form whatever the variant (scalar
+ * kernels on the fly: panels of 8 and 16 on the FP64 tensor-core path, everything else
+ * on the CUDA cores); a captured graph keeps the variant it was captured with.  No
+ * counterpart in the reference.
  */
 int h2gpu_set_jit_variant(h2gpu_image *img, int variant);
 
@@ -427,7 +429,9 @@ int h2gpu_pp_sketch_id(int kernel_id, const double *krnl_param, int n_krnl_param
  * L, both m x m, with the inverses of the triangular factor's 64 x 64 diagonal blocks, and
  * runs one launch per tree level per sweep (units of 64 rows over the whole GPU, which
  * wait for one another through bounded waits: H2GPU_ERR_DEVICE from the next call if one
- * expires; nodes of more than 13,872 rows are refused with H2GPU_ERR_UNSUPPORTED).
+ * expires).  A diagonal block that its inverse would not solve to the residual of
+ * substitution is solved by substitution.  Nodes of more than 13,872 rows, a fixed limit,
+ * are refused with H2GPU_ERR_UNSUPPORTED.
  */
 typedef struct h2gpu_ulv h2gpu_ulv;
 
