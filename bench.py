@@ -164,6 +164,9 @@ def run_reference(args):
     if rank != 0:
         return
     from oracle import oracle as O
+    if not O.have_ref():
+        print(json.dumps({"impl": "reference", "unavailable": "H2Pack's sources are not here: its library (oracle/_ref) is not built"}))
+        return
     cores = os.cpu_count()
     os.environ.setdefault("OMP_NUM_THREADS", str(cores))
     nv = args.nvec

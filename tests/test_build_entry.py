@@ -11,3 +11,15 @@ def test_build_without_h2pack_sources(monkeypatch, tmp_path, capsys):
     entry.build()
     assert made == [("h2pack_b200", ["libh2gpu.so"])]
     assert "libH2Pack_gpu.so" in capsys.readouterr().out
+
+
+def test_reference_arm_says_when_the_library_is_not_there(monkeypatch, capsys):
+    import json
+    import sys
+    import bench
+    from oracle import oracle
+    monkeypatch.setattr(oracle, "have_ref", lambda: False)
+    monkeypatch.setattr(sys, "argv", ["bench.py", "--impl", "reference", "--steps", "1", "--warmup", "1"])
+    bench.main()
+    line = json.loads(capsys.readouterr().out)
+    assert line["impl"] == "reference" and "not built" in line["unavailable"]
